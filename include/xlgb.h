@@ -134,14 +134,12 @@ enum {
 };
 /* Variants available for `pass` at transform length 2^log2_len (>= 1; 0 if
  * the pass or length is unknown).  Variant 0 is the default kernel shape
- * except at 4096 points: the RS column pass defaults to variant 8 (the
- * one-line kernel, persistent), the chirp-z x transform to variant 3
- * (registers sized for two CTAs per SM) and the chirp-z y transform to
- * variant 1 (persistent).  The others are the alternatives the autotuner
- * measures against the default.  RS column pass: 0 one line per thread,
- * 1-2 two lines per thread (packed FP32), 3-7 prefetching, barrier groups,
- * CTA shapes, 8 persistent one line, 9 (4096 points) radix 64, 10 (4096
- * points) as 8 with each unit's spectrum values kept in Tensor Memory.  Chirp-z x
+ * except at 4096 points: the chirp-z x transform defaults to variant 3
+ * (registers sized for two CTAs per SM), the chirp-z y transform to variant
+ * 1 (persistent) and the RS column pass to number 8.  The others are the
+ * alternatives the autotuner measures against the default.  RS column pass:
+ * every number selects the one kernel of that length (the numbers of kernels
+ * that earlier releases had are still accepted).  Chirp-z x
  * transform: 0 the stage capped for two CTAs per SM, 1 for one, 2 no
  * stage, 3 as 0 with registers for two CTAs, 4 (4096 points, three
  * components) one component group, two CTAs per SM.  Chirp-z y transform:

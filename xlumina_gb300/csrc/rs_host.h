@@ -24,6 +24,8 @@ struct RsLaunch {
   float2* work;
   XlProg pre, post;
   int adjoint;
+  int px;                       // columns of the intermediate (the x transform's length)
+  int lw;                       // log2 of its column-tile width
 };
 
 // Q = 2^logq is the half transform length: the smallest power of two >= the field side.

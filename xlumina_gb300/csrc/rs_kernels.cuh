@@ -35,8 +35,8 @@
 #include <type_traits>
 #include <vector>
 
-#include "fft64.cuh"
 #include "line_fft.cuh"
+#include "rs_blk.cuh"
 #include "rs_host.h"
 
 namespace xl {
@@ -359,305 +359,39 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
   }
 }
 
-// ---- Tensor Memory (tcgen05) as per-thread storage ----
-// TMEM is 128 lanes x 512 columns of 32-bit cells per SM.  With the 32x32b
-// access shape, thread i of warp w reads and writes lane 32 (w mod 4) + i, so
-// each thread owns its own cells; the kernels below give a thread 32
-// consecutive columns of its lane (16 complex values).  One warp allocates
-// the CTA's columns and hands the base address out through shared memory;
-// the same warp frees them before the CTA exits.
-__device__ __forceinline__ void tmem_alloc(unsigned* dst_smem, unsigned ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_fence_before_sync() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_fence_after_sync() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// four complex values into this thread's cells [col, col + 8)
-__device__ __forceinline__ void tmem_st4(unsigned taddr, float2 a, float2 b, float2 c, float2 d) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
-               "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// four complex values back; the values pass through the wait so that no use
-// is scheduled before the load has completed
-__device__ __forceinline__ void tmem_ld4(unsigned taddr, float2 (&o)[4]) {
-  float r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
-               : "r"(taddr)
-               : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7])
-               :
-               : "memory");
-#pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = make_float2(r[2 * i], r[2 * i + 1]);
-}
-
 // Column pass, in place on one tile of W spectrum columns: FFT along y of the
 // ny nonzero rows (pruned first pass), multiply by the transfer spectrum
 // (conjugate for the adjoint), inverse FFT, keep the ny surviving rows.
 // A CTA takes CW columns of a tile; lanes interleave them, so every warp
 // access is one contiguous run of CW columns.
-// L2 prefetch (PF): the CTA's spectrum columns at the start, and the next
-// component's column tile while this one is transformed, so that their loads
-// meet L2 rather than DRAM latency.
-// PERSIST: one CTA per resident slot walks the (batch entry, column group)
-// units batch entries fastest, as the grid does otherwise; the pass twiddle
-// table is then loaded once per CTA instead of once per unit.
-// TM (with PERSIST): the unit's spectrum values are read from global memory
-// for its first component only and kept in Tensor Memory for the others
-// (each thread's 16 values in its own TMEM cells), so the three components of
-// a VRS field read the spectrum tile from L2 once instead of three times.
-// The CTA allocates 256 of an SM's 512 TMEM columns; its shared memory allows
-// one such CTA per SM and no other kernel of the library allocates Tensor
-// Memory, so the allocation never has to wait for columns to be freed.
-template <int LOGQ, bool PF, bool PERSIST = false, bool TM = false>
+// Grid: batch entries fastest, so that the CTAs of one column tile run together
+// and share its transfer-spectrum columns in L2.
+template <int LOGQ>
 __global__ void __launch_bounds__(RsCfg<LOGQ>::COL_THREADS, RsCfg<LOGQ>::COL_MINB)
     rs_cols_conv(const __grid_constant__ RsLaunch p) {
   using C = RsCfg<LOGQ>;
   constexpr int W = C::W, CW = C::CW, LPW = 32 / CW;
-  // TMEM columns: 32 per thread, the warps of a lane quarter side by side
-  constexpr unsigned TM_COLS = (unsigned)(C::COL_THREADS / 128) * 32u;
-  static_assert(!TM || (PERSIST && C::COL_THREADS % 128 == 0 && TM_COLS >= 32 && TM_COLS <= 256 &&
-                        (TM_COLS & (TM_COLS - 1)) == 0),
-                "TMEM spectrum cache: persistent CTAs of whole warp quarters, a power-of-two column count");
   extern __shared__ __align__(16) float2 smem[];
-  __shared__ unsigned s_tmem;
   float2* xch = smem;                  // CW x CXS
   float2* stw = smem + CW * C::CXS;    // NTW
   const int tid = threadIdx.x, lane = tid & 31;
   const int wc = lane % CW, j = (tid >> 5) * LPW + lane / CW;
-  if constexpr (TM) {
-    if (tid < 32) tmem_alloc(&s_tmem, TM_COLS);
-  }
   {
     const float2* g = pass_tw<C::LOGP>();
     for (int i = tid; i < C::NTW; i += blockDim.x) stw[i] = g[i];
   }
-  if constexpr (TM) tmem_fence_before_sync();
   __syncthreads();
-  unsigned tcell = 0;   // this thread's first TMEM cell: lane 32 (warp mod 4) + lane, 32 columns per warp
-  if constexpr (TM) {
-    tmem_fence_after_sync();
-    tcell = s_tmem + ((32u * ((unsigned)(tid >> 5) & 3u)) << 16) + (unsigned)(tid >> 7) * 32u;
-  }
   float2* xb = xch + wc * C::CXS;
   const int ny = p.ny;
-  const int units = PERSIST ? p.B * (C::P / CW) : 1;
-#pragma unroll 1
-  for (int u = PERSIST ? (int)blockIdx.x : 0; u < units; u += PERSIST ? (int)gridDim.x : 1) {
-    // batch entries fastest: the CTAs of one column tile run together and share
-    // its transfer-spectrum columns in L2
-    const int b = PERSIST ? u % p.B : (int)blockIdx.x;
-    const int g = PERSIST ? u / p.B : (int)blockIdx.y;
-    const int t = g / (W / CW);                      // column tile
-    const int w = (g % (W / CW)) * CW + wc;          // column within the tile
-    const int kx = t * W + w;
-    const float2* sbase = p.specs ? p.specs[b] : p.spec + (long long)(p.sidx ? p.sidx[b] : 0) * p.sstride;
-    const float2* spec = sbase + (long long)(kx / C::SW) * C::P * C::SW + kx % C::SW;
-    if (PF && tid == 0) l2_prefetch(sbase + (long long)(kx / C::SW) * C::P * C::SW, (unsigned)(C::P * C::SW * 8));
-#pragma unroll 1
-    for (int c = 0; c < p.cout; ++c) {
-      float2* tile = p.work + ((long long)b * p.cout + c) * ny * C::P + (long long)t * ny * W + w;
-      if (PF && tid == 0 && c + 1 < p.cout)
-        l2_prefetch(p.work + ((long long)b * p.cout + c + 1) * ny * C::P + (long long)t * ny * W,
-                    (unsigned)(ny * W * 8));
-      float2 v[16];
-#pragma unroll
-      for (int m = 0; m < C::H; ++m) {
-        const int n = j + m * C::T;
-        v[m] = n < ny ? tile[(long long)n * W] : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int m = C::H; m < 16; ++m) v[m] = make_float2(0.f, 0.f);
-      block_fft_x<C::LOGP, 16, -1, true, false>(v, j, xb, stw);
-      // the spectrum loads stay here rather than ahead of the transform, where
-      // they would hold 32 registers through it
-      if (TM && c > 0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 s[4];
-          tmem_ld4(tcell + 8u * q, s);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) v[4 * q + i] = p.adjoint ? cmulc(v[4 * q + i], s[i]) : cmul(v[4 * q + i], s[i]);
-        }
-      } else if (TM) {
-        const float2* sp = spec;
-        asm volatile("" : "+l"(sp));
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float2 s[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s[i] = __ldg(sp + (long long)(j + (4 * q + i) * C::T) * C::SW);
-          tmem_st4(tcell + 8u * q, s[0], s[1], s[2], s[3]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) v[4 * q + i] = p.adjoint ? cmulc(v[4 * q + i], s[i]) : cmul(v[4 * q + i], s[i]);
-        }
-        tmem_wait_st();   // the stores are complete before the next component's loads
-      } else {
-        const float2* sp = spec;
-        asm volatile("" : "+l"(sp));
-        if (p.adjoint) {
-#pragma unroll
-          for (int m = 0; m < 16; ++m) v[m] = cmulc(v[m], __ldg(sp + (long long)(j + m * C::T) * C::SW));
-        } else {
-#pragma unroll
-          for (int m = 0; m < 16; ++m) v[m] = cmul(v[m], __ldg(sp + (long long)(j + m * C::T) * C::SW));
-        }
-      }
-      block_fft_x<C::LOGP, 16, 1, false, false>(v, j, xb, stw);
-#pragma unroll
-      for (int m = 0; m < C::H; ++m) {
-        const int n = j + m * C::T;
-        if (n < ny) tile[(long long)n * W] = v[m];
-      }
-    }
-  }
-  if constexpr (TM) {
-    // every thread is done with its cells before the allocating warp frees them
-    tmem_fence_before_sync();
-    __syncthreads();
-    if (tid < 32) {
-      tmem_fence_after_sync();
-      tmem_dealloc(s_tmem, TM_COLS);
-    }
-  }
-}
-
-// Column pass at P = 4096 with the radix-64 engine (fft64.cuh): 64 threads
-// per column hold 64 elements each, so a transform has one exchange instead
-// of two and the CTA (4 columns, 256 threads, one per SM) runs four barriers
-// per component instead of eight.  Persistent: each CTA builds the pass-0
-// twiddle table once and walks (batch entry, column group) units batch
-// entries fastest, as the one-line kernel's grid does.
-template <int LOGQ>
-__global__ void __launch_bounds__(256, 1) rs_cols_conv64(const __grid_constant__ RsLaunch p) {
-  using C = RsCfg<LOGQ>;
-  static_assert(C::P == 4096 && C::CW == 4, "radix-64 column pass: P = 4096, 4 columns per CTA");
-  constexpr int W = C::W, CW = C::CW;
-  extern __shared__ __align__(16) float2 smem[];
-  float2* xch = smem;                    // CW lines, F64_XB slots apart
-  float2* stw = smem + CW * F64_XB;      // 4096: w4096^(j k) at k * 64 + j
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int wc = lane & 3, j = (tid >> 5) * 8 + (lane >> 2);
-  {
-    const float2* g = tw_table(12);
-    for (int i = tid; i < 4096; i += 256) stw[i] = f64_twiddle_entry(i, g);
-  }
-  float2* xb = xch + wc * F64_XB;
-  const int ny = p.ny;
-  const int units = p.B * (C::P / CW);
-#pragma unroll 1
-  for (int u = blockIdx.x; u < units; u += gridDim.x) {
-    const int b = u % p.B, grp = u / p.B;
-    const int t = grp / (W / CW);                      // column tile
-    const int w = (grp % (W / CW)) * CW + wc;          // column within the tile
-    const int kx = t * W + w;
-    const float2* sbase = p.specs ? p.specs[b] : p.spec + (long long)(p.sidx ? p.sidx[b] : 0) * p.sstride;
-    const float2* spec = sbase + (long long)(kx / C::SW) * C::P * C::SW + kx % C::SW;
-#pragma unroll 1
-    for (int c = 0; c < p.cout; ++c) {
-      float2* tile = p.work + ((long long)b * p.cout + c) * ny * C::P + (long long)t * ny * W + w;
-      float2 v[64];
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int n = j + 64 * m;
-        v[m] = n < ny ? tile[(long long)n * W] : make_float2(0.f, 0.f);
-      }
-      f64_pass0<-1, true>(v);
-      __syncthreads();   // the previous transform's gathers are done (and the table is built)
-      f64_write<-1>(v, j, xb, stw);
-      __syncthreads();
-      f64_pass1<-1, false>(v, j, xb);
-      const float2* sp = spec;
-      asm volatile("" : "+l"(sp));
-      if (p.adjoint) {
-#pragma unroll
-        for (int m = 0; m < 64; ++m) v[m] = cmulc(v[m], __ldg(sp + (long long)(j + 64 * m) * C::SW));
-      } else {
-#pragma unroll
-        for (int m = 0; m < 64; ++m) v[m] = cmul(v[m], __ldg(sp + (long long)(j + 64 * m) * C::SW));
-      }
-      f64_pass0<1, false>(v);
-      __syncthreads();
-      f64_write<1>(v, j, xb, stw);
-      __syncthreads();
-      f64_pass1<1, true>(v, j, xb);
-#pragma unroll
-      for (int m = 0; m < 32; ++m) {
-        const int n = j + 64 * m;
-        if (n < ny) tile[(long long)n * W] = v[m];
-      }
-    }
-  }
-}
-
-// One-line column pass in other CTA shapes: CWK columns per CTA (CWK = CW:
-// one CTA per SM; CWK = CW / 2: two), split into NGRP groups of CWK / NGRP
-// columns with their own named barriers, so that groups (or co-resident CTAs)
-// in different phases overlap one's exchanges with another's arithmetic.
-// With L2 prefetch of the spectrum and of the next component's tile.
-template <int LOGQ, int CWK, int NGRP> struct RsColShape {
-  using C = RsCfg<LOGQ>;
-  static constexpr int CWG = CWK / NGRP;                  // columns per group
-  static constexpr int THREADS = CWK * C::T;
-  static constexpr int MINB = (1024 / THREADS) > 1 ? (1024 / THREADS) : 1;
-  static constexpr int XSK = C::XS + (CWG >= 8 ? 0 : 16 / CWG);
-  static constexpr size_t SMEM = ((size_t)CWK * XSK + C::NTW) * sizeof(float2);
-  static_assert(C::CW % CWK == 0 && CWK % NGRP == 0 && (CWG * C::T) % 32 == 0, "column CTA shape");
-};
-
-// STAGGER (two groups): group 1 starts its first component only once group 0
-// has finished that component's forward transform, so that the groups run
-// half a component apart and one's loads and exchanges meet the other's
-// arithmetic instead of its own.
-template <int LOGQ, int CWK, int NGRP, bool STAGGER = false>
-__global__ void __launch_bounds__(RsColShape<LOGQ, CWK, NGRP>::THREADS, RsColShape<LOGQ, CWK, NGRP>::MINB)
-    rs_cols_conv_g(const __grid_constant__ RsLaunch p) {
-  using C = RsCfg<LOGQ>;
-  using K = RsColShape<LOGQ, CWK, NGRP>;
-  constexpr int W = C::W, CWG = K::CWG, LPW = 32 / CWG;
-  extern __shared__ __align__(16) float2 smem[];
-  float2* stw = smem + CWK * K::XSK;
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int grp = tid / (CWG * C::T), gtid = tid % (CWG * C::T);
-  const int wc = lane % CWG, j = (gtid >> 5) * LPW + lane / CWG;
-  const int t = blockIdx.y / (W / CWK);
-  const int w = (blockIdx.y % (W / CWK)) * CWK + grp * CWG + wc;
-  const int b = blockIdx.x;
-  const int ny = p.ny;
-  {
-    const float2* g = pass_tw<C::LOGP>();
-    for (int i = tid; i < C::NTW; i += blockDim.x) stw[i] = g[i];
-  }
-  __syncthreads();
+  const int b = (int)blockIdx.x, g = (int)blockIdx.y;
+  const int t = g / (W / CW);                      // column tile
+  const int w = (g % (W / CW)) * CW + wc;          // column within the tile
   const int kx = t * W + w;
   const float2* sbase = p.specs ? p.specs[b] : p.spec + (long long)(p.sidx ? p.sidx[b] : 0) * p.sstride;
   const float2* spec = sbase + (long long)(kx / C::SW) * C::P * C::SW + kx % C::SW;
-  float2* xb = smem + (grp * CWG + wc) * K::XSK;
-  using Sync = typename std::conditional<(NGRP > 1), GroupSync, CtaSync>::type;
-  Sync sync;
-  if constexpr (NGRP > 1) sync = GroupSync{1 + grp, CWG * C::T};
-  if (tid == 0) l2_prefetch(sbase + (long long)(kx / C::SW) * C::P * C::SW, (unsigned)(C::P * C::SW * 8));
-  if constexpr (STAGGER && NGRP == 2) {
-    if (grp == 1) asm volatile("bar.sync 3, %0;" ::"r"(K::THREADS) : "memory");
-  }
 #pragma unroll 1
   for (int c = 0; c < p.cout; ++c) {
-    const long long tbase = ((long long)b * p.cout + c) * ny * C::P + (long long)t * ny * W;
-    float2* tile = p.work + tbase + w;
-    if (tid == 0 && c + 1 < p.cout) l2_prefetch(p.work + tbase + (long long)ny * C::P, (unsigned)(ny * W * 8));
+    float2* tile = p.work + ((long long)b * p.cout + c) * ny * C::P + (long long)t * ny * W + w;
     float2 v[16];
 #pragma unroll
     for (int m = 0; m < C::H; ++m) {
@@ -666,10 +400,9 @@ __global__ void __launch_bounds__(RsColShape<LOGQ, CWK, NGRP>::THREADS, RsColSha
     }
 #pragma unroll
     for (int m = C::H; m < 16; ++m) v[m] = make_float2(0.f, 0.f);
-    block_fft_x<C::LOGP, 16, -1, true, false>(v, j, xb, stw, sync);
-    if constexpr (STAGGER && NGRP == 2) {
-      if (grp == 0 && c == 0) asm volatile("bar.arrive 3, %0;" ::"r"(K::THREADS) : "memory");
-    }
+    block_fft_x<C::LOGP, 16, -1, true, false>(v, j, xb, stw);
+    // the spectrum loads stay here rather than ahead of the transform, where
+    // they would hold 32 registers through it
     const float2* sp = spec;
     asm volatile("" : "+l"(sp));
     if (p.adjoint) {
@@ -679,119 +412,11 @@ __global__ void __launch_bounds__(RsColShape<LOGQ, CWK, NGRP>::THREADS, RsColSha
 #pragma unroll
       for (int m = 0; m < 16; ++m) v[m] = cmul(v[m], __ldg(sp + (long long)(j + m * C::T) * C::SW));
     }
-    block_fft_x<C::LOGP, 16, 1, false, false>(v, j, xb, stw, sync);
+    block_fft_x<C::LOGP, 16, 1, false, false>(v, j, xb, stw);
 #pragma unroll
     for (int m = 0; m < C::H; ++m) {
       const int n = j + m * C::T;
       if (n < ny) tile[(long long)n * W] = v[m];
-    }
-  }
-}
-
-// Column pass on the packed two-line engine (fft_pair.cuh): each thread
-// transforms two adjacent columns of the CTA's CW at once, so every butterfly
-// instruction works on both, and loads, stores and exchanges move the two
-// columns' elements as one 16-byte access.  NG = CW / 2 column pairs per CTA.
-// GROUPED: pair g is a group of T threads (whole warps) with its own named
-// barrier, so the groups drift apart and one group's loads overlap another's
-// arithmetic; otherwise the pairs interleave in the lanes of every warp (a
-// warp load covers whole 32-byte sectors) under one CTA barrier.
-template <int LOGQ, bool GROUPED> struct RsColPair {
-  using C = RsCfg<LOGQ>;
-  static constexpr int NG = C::CW / 2;
-  static constexpr int THREADS = NG * C::T;
-  // pair buffers offset by 8 / NG slots mod 8 when the pairs share a warp, so
-  // that one quarter-warp's 16-byte accesses fall in distinct banks
-  static constexpr int XSP = C::XS + (GROUPED ? 0 : 8 / NG);
-  static constexpr size_t SMEM = ((size_t)NG * XSP + C::NTW) * 16;
-  static constexpr int MINB = (512 / THREADS) > 1 ? (512 / THREADS) : 1;   // at most 128 registers
-  static_assert(C::CW % 2 == 0 && C::T % 32 == 0, "two-line column pass shape");
-  static_assert(GROUPED || (32 % NG == 0 && C::T % (32 / NG) == 0), "interleaved lanes");
-};
-
-// PF: L2 prefetch as in rs_cols_conv; RP: the next component's inputs are
-// loaded into registers at the start of this component's transforms, so their
-// latency is spent under the arithmetic.
-template <int LOGQ, bool GROUPED, bool PF = false, bool RP = false>
-__global__ void __launch_bounds__(RsColPair<LOGQ, GROUPED>::THREADS, RsColPair<LOGQ, GROUPED>::MINB)
-    rs_cols_conv_p(const __grid_constant__ RsLaunch p) {
-  using C = RsCfg<LOGQ>;
-  using K = RsColPair<LOGQ, GROUPED>;
-  constexpr int W = C::W, CW = C::CW, NG = K::NG;
-  extern __shared__ __align__(16) float4 smem4[];
-  float4* stw = smem4 + NG * K::XSP;   // NTW pair twiddles
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int pr = GROUPED ? tid / C::T : lane % NG;
-  const int j = GROUPED ? tid % C::T : (tid >> 5) * (32 / NG) + lane / NG;
-  const int t = blockIdx.y / (W / CW);                       // column tile
-  const int w = (blockIdx.y % (W / CW)) * CW + 2 * pr;       // first column of the pair within the tile
-  const int b = blockIdx.x;
-  const int ny = p.ny;
-  {
-    const float4* g = pass_tw4<C::LOGP>();
-    for (int i = tid; i < C::NTW; i += blockDim.x) stw[i] = g[i];
-  }
-  __syncthreads();
-  const int kx = t * W + w;
-  const float2* sbase = p.specs ? p.specs[b] : p.spec + (long long)(p.sidx ? p.sidx[b] : 0) * p.sstride;
-  const float2* spec = sbase + (long long)(kx / C::SW) * C::P * C::SW + kx % C::SW;
-  float4* xb = smem4 + pr * K::XSP;
-  using Sync = typename std::conditional<GROUPED, GroupSync, CtaSync>::type;
-  Sync sync;
-  if constexpr (GROUPED) sync = GroupSync{1 + pr, C::T};
-  auto tile_of = [&](int c) {
-    return p.work + ((long long)b * p.cout + c) * ny * C::P + (long long)t * ny * W + w;
-  };
-  auto load_in = [&](int c, float4 (&dst)[C::H]) {
-    const float2* tl = tile_of(c);
-#pragma unroll
-    for (int m = 0; m < C::H; ++m) {
-      const int n = j + m * C::T;
-      dst[m] = n < ny ? *(const float4*)(tl + (long long)n * W) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  if (PF && tid == 0) l2_prefetch(sbase + (long long)(kx / C::SW) * C::P * C::SW, (unsigned)(C::P * C::SW * 8));
-  float4 nxt[RP ? C::H : 1];
-  if constexpr (RP) load_in(0, nxt);
-#pragma unroll 1
-  for (int c = 0; c < p.cout; ++c) {
-    float2* tile = tile_of(c);
-    if (PF && tid == 0 && c + 1 < p.cout) l2_prefetch(tile_of(c + 1) - w, (unsigned)(ny * W * 8));
-    cpair v[16];
-    if constexpr (RP) {
-#pragma unroll
-      for (int m = 0; m < C::H; ++m) v[m] = p_from(nxt[m]);
-      if (c + 1 < p.cout) load_in(c + 1, nxt);
-    } else {
-#pragma unroll
-      for (int m = 0; m < C::H; ++m) {
-        const int n = j + m * C::T;
-        v[m] = n < ny ? p_from(*(const float4*)(tile + (long long)n * W)) : pz();
-      }
-    }
-#pragma unroll
-    for (int m = C::H; m < 16; ++m) v[m] = pz();
-    block_pfft<C::LOGP, -1, true, false>(v, j, xb, stw, sync);
-    const float2* sp = spec;
-    asm volatile("" : "+l"(sp));
-    if (p.adjoint) {
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const float4 s = __ldg((const float4*)(sp + (long long)(j + m * C::T) * C::SW));
-        v[m] = pmul_pp<true>(v[m], make_float2(s.x, s.z), make_float2(s.y, s.w));
-      }
-    } else {
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const float4 s = __ldg((const float4*)(sp + (long long)(j + m * C::T) * C::SW));
-        v[m] = pmul_pp<false>(v[m], make_float2(s.x, s.z), make_float2(s.y, s.w));
-      }
-    }
-    block_pfft<C::LOGP, 1, false, false>(v, j, xb, stw, sync);
-#pragma unroll
-    for (int m = 0; m < C::H; ++m) {
-      const int n = j + m * C::T;
-      if (n < ny) *(float4*)(tile + (long long)n * W) = p_to(v[m]);
     }
   }
 }
@@ -926,11 +551,15 @@ int rs_spectrum(cudaStream_t st, int ny, int nx, const double* offx, const doubl
                                                                            k, work);
   }
   XL_CHECK_LAUNCH("rs_hhat_rows");
-  const size_t sm2 = (size_t)C::CW * C::CXS * sizeof(float2);
-  e = allow_smem(rs_hhat_cols<LOGQ>, sm2);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols smem");
-  rs_hhat_cols<LOGQ><<<C::P / C::CW, C::COL_THREADS, sm2, st>>>(work, (float)scale, spec);
-  XL_CHECK_LAUNCH("rs_hhat_cols");
+  if constexpr (LOGQ >= 9 && LOGQ <= 11) {
+    return launch_hhat_cols_b<C::P / 256>(st, work, C::P, (float)scale, spec);
+  } else {
+    const size_t sm2 = (size_t)C::CW * C::CXS * sizeof(float2);
+    e = allow_smem(rs_hhat_cols<LOGQ>, sm2);
+    if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols smem");
+    rs_hhat_cols<LOGQ><<<C::P / C::CW, C::COL_THREADS, sm2, st>>>(work, (float)scale, spec);
+    XL_CHECK_LAUNCH("rs_hhat_cols");
+  }
   return XL_OK;
 }
 
@@ -975,52 +604,13 @@ static int launch_rows_inv(cudaStream_t s, const RsLaunch& p) {
   return XL_OK;
 }
 
-template <int LOGQ, bool GROUPED, bool PF = false, bool RP = false>
-static int launch_cols_pair(cudaStream_t st, const RsLaunch& p) {
-  using C = RsCfg<LOGQ>;
-  using K = RsColPair<LOGQ, GROUPED>;
-  cudaError_t e = allow_smem(rs_cols_conv_p<LOGQ, GROUPED, PF, RP>, K::SMEM);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_cols_conv_p smem");
-  rs_cols_conv_p<LOGQ, GROUPED, PF, RP><<<dim3(p.B, C::P / C::CW), K::THREADS, K::SMEM, st>>>(p);
-  XL_CHECK_LAUNCH("rs_cols_conv_p");
-  return XL_OK;
-}
-
-template <int LOGQ, int CWK, int NGRP, bool STAGGER = false>
-static int launch_cols_g(cudaStream_t st, const RsLaunch& p) {
-  using C = RsCfg<LOGQ>;
-  using K = RsColShape<LOGQ, CWK, NGRP>;
-  cudaError_t e = allow_smem(rs_cols_conv_g<LOGQ, CWK, NGRP, STAGGER>, K::SMEM);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_cols_conv_g smem");
-  rs_cols_conv_g<LOGQ, CWK, NGRP, STAGGER><<<dim3(p.B, C::P / CWK), K::THREADS, K::SMEM, st>>>(p);
-  XL_CHECK_LAUNCH("rs_cols_conv_g");
-  return XL_OK;
-}
-
 template <int LOGQ>
-static int launch_cols64(cudaStream_t st, const RsLaunch& p) {
-  using C = RsCfg<LOGQ>;
-  const size_t sm = (size_t)(C::CW * F64_XB + 4096) * sizeof(float2);
-  cudaError_t e = allow_smem(rs_cols_conv64<LOGQ>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_cols_conv64 smem");
-  const int grid = persistent_grid(rs_cols_conv64<LOGQ>, 256, sm, p.B * (C::P / C::CW));
-  rs_cols_conv64<LOGQ><<<grid, 256, sm, st>>>(p);
-  XL_CHECK_LAUNCH("rs_cols_conv64");
-  return XL_OK;
-}
-
-template <int LOGQ, bool PF, bool PERSIST = false, bool TM = false>
 static int launch_cols(cudaStream_t st, const RsLaunch& p) {
   using C = RsCfg<LOGQ>;
   const size_t sm = (size_t)(C::CW * C::CXS + C::NTW) * sizeof(float2);
-  cudaError_t e = allow_smem(rs_cols_conv<LOGQ, PF, PERSIST, TM>, sm);
+  cudaError_t e = allow_smem(rs_cols_conv<LOGQ>, sm);
   if (e != cudaSuccess) return cuda_fail(e, "rs_cols_conv smem");
-  if constexpr (PERSIST) {
-    const int grid = persistent_grid(rs_cols_conv<LOGQ, PF, true, TM>, C::COL_THREADS, sm, p.B * (C::P / C::CW));
-    rs_cols_conv<LOGQ, PF, true, TM><<<grid, C::COL_THREADS, sm, st>>>(p);
-  } else {
-    rs_cols_conv<LOGQ, PF><<<dim3(p.B, C::P / C::CW), C::COL_THREADS, sm, st>>>(p);
-  }
+  rs_cols_conv<LOGQ><<<dim3(p.B, C::P / C::CW), C::COL_THREADS, sm, st>>>(p);
   XL_CHECK_LAUNCH("rs_cols_conv");
   return XL_OK;
 }
@@ -1046,24 +636,8 @@ static int launch_stage(cudaStream_t st, const RsLaunch& p, int stage) {
     }
     return launch_rows_fwd<LOGQ, 3>(st, p);
   } else if (stage == 1) {
-    const int var = kernel_variant(XL_PASS_RS_COLS, C::LOGP);
-    if constexpr (LOGQ >= 9 && LOGQ <= 11) {
-      if (var == 1) return launch_cols_pair<LOGQ, false>(st, p);
-      if (var == 2) return launch_cols_pair<LOGQ, true>(st, p);
-      if (var == 3) return launch_cols<LOGQ, true>(st, p);
-      if (var == 4) return launch_cols_pair<LOGQ, false, true, true>(st, p);
-      if (var == 5) return launch_cols_g<LOGQ, C::CW, 2>(st, p);
-      if (var == 6) return launch_cols_g<LOGQ, C::CW / 2, 1>(st, p);
-      if (var == 7) return launch_cols_g<LOGQ, C::CW, 2, true>(st, p);
-    }
-    if constexpr (LOGQ >= 9 && LOGQ <= 11) {
-      if (var == 8) return launch_cols<LOGQ, false, true>(st, p);
-    }
-    if constexpr (LOGQ == 11) {
-      if (var == 9) return launch_cols64<LOGQ>(st, p);
-      if (var == 10) return launch_cols<LOGQ, false, true, true>(st, p);
-    }
-    return launch_cols<LOGQ, false>(st, p);
+    if constexpr (LOGQ >= 9 && LOGQ <= 11) return launch_cols_b<C::P / 256>(st, p);
+    else return launch_cols<LOGQ>(st, p);
   } else {
     const bool epi = p.post.nops > 0 || (p.adjoint && p.cout == 3);
     if (p.cout == 1) return epi ? launch_rows_inv<LOGQ, 1, true>(st, p) : launch_rows_inv<LOGQ, 1, false>(st, p);
@@ -1073,7 +647,10 @@ static int launch_stage(cudaStream_t st, const RsLaunch& p, int stage) {
 }
 
 template <int LOGQ>
-int rs_propagate(cudaStream_t st, const RsLaunch& p, int stage) {
+int rs_propagate(cudaStream_t st, const RsLaunch& q, int stage) {
+  RsLaunch p = q;
+  p.px = RsCfg<LOGQ>::P;
+  p.lw = RsCfg<LOGQ>::W == 8 ? 3 : (RsCfg<LOGQ>::W == 4 ? 2 : 1);
   if (stage >= 0) return launch_stage<LOGQ>(st, p, stage);
   for (int s = 0; s < 3; ++s)
     if (int rc = launch_stage<LOGQ>(st, p, s)) return rc;
