@@ -1,0 +1,5 @@
+// RS / VRS passes of 2560-point transforms on the block FFT engine (one
+// translation unit of rs_blk.cuh).
+#include "rs_blk.cuh"
+
+XL_RS_BLK_INSTANTIATE(10)

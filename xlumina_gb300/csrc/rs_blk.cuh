@@ -2,7 +2,11 @@
 // transforms of P = 256 R points.
 #pragma once
 
+#include <math.h>
+
 #include <type_traits>
+#include <vector>
+
 #include "fft_block.cuh"
 #include "line_fft.cuh"
 #include "rs_host.h"
@@ -79,15 +83,19 @@ __device__ __forceinline__ void tmem_ld4(unsigned taddr, float2 (&o)[4]) {
 }
 
 // Column CTAs: CW columns, interleaved in the lanes of phase A (a warp's load
-// or store of a row is then a whole 32-byte sector), T threads each.
+// or store of a row is then whole 32-byte sectors), T threads each.  CW = 8
+// fills a CTA of 1024 threads where a line takes 128 (8 x 1024^2 VRS adjoint:
+// 378 us, with two CTAs of 4 columns an SM 403); where a line takes 64, four
+// CTAs of 4 columns an SM are the better form (16 x 500^2 VRS: 184 us, two of
+// 8 columns 193).
 template <int R> struct RsColB {
   using F = BlkFft<R>;
-  static constexpr int CW = 4, LPW = 32 / CW;
+  static constexpr int CW = F::T == 128 ? 8 : 4, LPW = 32 / CW;
   static constexpr int THREADS = CW * F::T;
   static constexpr int MINB = 1024 / THREADS;
-  static constexpr int LINE = F::LINE + 4;     // the CW columns of a half-warp on distinct banks
+  static constexpr int LINE = F::LINE + 16 / CW;   // the CW columns of a half-warp on distinct banks
   static constexpr int WARPS_B = CW * R / 2;   // warps of phases B and C
-  static constexpr bool TM = R > 8;            // Tensor Memory cells beside the registers
+  static constexpr bool TM = MINB == 1;        // Tensor Memory cells beside the registers
   static constexpr unsigned TM_COLS = THREADS / 128 * 64;
   static constexpr size_t SMEM = ((size_t)F::NTW + (size_t)CW * LINE) * 8;
 };
@@ -114,7 +122,7 @@ template <int R> struct ColMap {
 // FFT, keep the ny surviving rows.  Persistent: CTAs walk the (batch entry,
 // column group) units batch entries fastest, so that entries at the same
 // distance read one spectrum tile together.  Spectra are stored in the order
-// phase C holds them (rs_hhat_cols_b), so a warp reads 512 contiguous bytes.
+// phase C holds them (rs_hhat_cols_b), so a warp reads 256 contiguous bytes.
 // Phase A twiddles, four at a time, from this thread's Tensor Memory cells or
 // from the table in shared memory.
 template <int R> struct TmemTw {
@@ -136,18 +144,17 @@ template <int R> struct SmemTw {
 // FFT, keep the ny surviving rows.  Persistent: CTAs walk the (batch entry,
 // column group) units batch entries fastest, so that entries at the same
 // distance read one spectrum tile together.  Spectra are stored in the order
-// phase C holds them (rs_hhat_cols_b), so a warp reads 512 contiguous bytes.
+// phase C holds them (rs_hhat_cols_b), so a warp reads 256 contiguous bytes.
 //
 // What bounds it: the shared-memory pipe (60 % busy at 4096 points, the FP32
 // pipe 48 %); without any of its global loads and stores it runs 16 % faster.
-// So the CTAs of 1024 threads (R > 8) keep what a thread reads again and again
+// So the CTAs of 1024 threads (R > 4) keep what a thread reads again and again
 // in its own Tensor Memory cells, which are not on that pipe: the phase A
 // twiddles (a thread's j never changes), and a unit's spectrum values for the
 // second and third component.  8 x 2048^2 VRS: 1.50 ms with both, 1.58 ms
 // without, 1.92 ms on the Stockham engine with its eight barriers a component.
-// The smaller CTAs (R <= 8, several per SM) keep their tables in shared
-// memory: with Tensor Memory they ran a third slower (16 x 1024^2 scalar: 339
-// against 250 us; Stockham 313 us).
+// The smaller CTAs (R = 4, four per SM) keep their tables in shared memory: with
+// Tensor Memory they took 291 against 178 us for 16 x 500^2 VRS.
 //
 // A thread holds 64 of the Tensor Memory columns of its lane, CTAs of 1024
 // threads all 512; the 64 registers of a thread allow one such CTA per SM, so
@@ -200,7 +207,7 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
     const int b = u % p.B, g = u / p.B;
     const long long col = (long long)g * K::CW + m.wc;
     const float2* sbase = p.specs ? p.specs[b] : p.spec + (long long)(p.sidx ? p.sidx[b] : 0) * p.sstride;
-    const float4* spec = (const float4*)sbase + (long long)g * (K::CW * F::P / 2) + m.warp * 256 + m.lane;
+    const float2* spec = sbase + (long long)g * (K::CW * F::P) + m.warp * 512 + m.lane;
 #pragma unroll 1
     for (int c = 0; c < p.cout; ++c) {
       float2* tile = p.work + ((long long)b * p.cout + c) * ny * p.px + (((col >> lw) * ny) << lw) +
@@ -219,7 +226,7 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
         blk_b_fwd<-1>(v, m.l, blk, twb);
         __syncwarp();
         blk_c_fwd<-1>(v, m.l, blk);
-        const float4* sp = spec;
+        const float2* sp = spec;
         asm volatile("" : "+l"(sp));   // the loads stay here: ahead of the transform they would hold 32 registers
         auto mul4 = [&](int q, const float2 (&w)[4]) {
 #pragma unroll
@@ -235,9 +242,9 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
         } else {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float4 s = __ldg(sp + 2 * q * 32), t = __ldg(sp + (2 * q + 1) * 32);
-            const float2 w[4] = {make_float2(s.x, s.y), make_float2(s.z, s.w), make_float2(t.x, t.y),
-                                 make_float2(t.z, t.w)};
+            float2 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = __ldg(sp + (4 * q + i) * 32);
             if (TM && p.cout > 1) tmem_st4(scell + 8u * q, w[0], w[1], w[2], w[3]);
             mul4(q, w);
           }
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
 
 // Transfer spectrum, column transforms of the row spectra (`in`: P rows of px
 // columns), times `scale`, stored per group of CW columns in the order phase
-// C of the column pass holds them: [group][warp][register pair][lane][2].
+// C of the column pass holds them: [group][warp][register][lane].
 template <int R>
 __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB)
     rs_hhat_cols_b(const float2* __restrict__ in, int px, float scale, float2* __restrict__ out) {
@@ -299,11 +306,491 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB)
   blk_b_fwd<-1>(v, m.l, blk, tw + F::NTA);
   __syncwarp();
   blk_c_fwd<-1>(v, m.l, blk);
-  float4* dst = (float4*)out + (long long)blockIdx.x * (K::CW * F::P / 2) + m.warp * 256 + m.lane;
+  float2* dst = out + (long long)blockIdx.x * (K::CW * F::P) + m.warp * 512 + m.lane;
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    dst[q * 32] = make_float4(v[2 * q].x * scale, v[2 * q].y * scale, v[2 * q + 1].x * scale, v[2 * q + 1].y * scale);
+  for (int q = 0; q < 16; ++q) dst[32 * q] = cscale(v[q], scale);
 }
+
+// ---- row passes ----
+// Positions: the P columns of the intermediate are in the order the row
+// passes' phase C threads hold them: thread (k1, k2) = warp wq, lane of its
+// line holds register m at position (wq 16 + m) 32 + lane, so a warp's access
+// covers 32 positions.  Column groups and transfer spectra are in the same
+// order.
+
+// Thread organisation for NC transformed components: CG component groups of G
+// lines of T threads, where CG = NC (every component of a row transformed at
+// once) when the CTA can hold them, else 1 (one after the other).
+template <int R, int NC> struct RowB {
+  using F = BlkFft<R>;
+  static constexpr int G = 256 / F::T > 1 ? 256 / F::T : 1;
+  static constexpr int CG = (NC * G * F::T <= 1024) ? NC : 1;
+  static constexpr int LINES = CG * G;
+  static constexpr int THREADS = LINES * F::T;
+  static constexpr int MINB = (768 / THREADS) > 1 ? (768 / THREADS) : 1;   // resident CTAs per SM
+  static constexpr bool TM = MINB == 1;       // phase A twiddles in Tensor Memory
+};
+
+// Phase A twiddles of a row thread: the table in global memory, the same
+// entries on every row.
+template <int R> struct GlobalTw {
+  const float2* tw;   // the table at the thread's j
+  __device__ __forceinline__ void operator()(int i, int q, float2 (&w)[4]) const {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+      if (4 * q + n > 0 && 4 * q + n < R) w[n] = __ldg(tw + (4 * q + n - 1) * 256 + i * BlkFft<R>::T);
+  }
+};
+
+// The same entries in Tensor Memory, 32 cells a thread: allocates for a CTA of
+// THREADS threads, fills, and returns the thread's first cell.
+template <int THREADS> constexpr unsigned tmem_cols32() {
+  unsigned n = 32;
+  while (n < (THREADS + 127) / 128 * 32u) n *= 2;
+  return n;
+}
+template <int R, int THREADS, class TW> __device__ __forceinline__ unsigned tmem_twiddles(unsigned* s_tmem, const TW& tw) {
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) tmem_alloc(s_tmem, tmem_cols32<THREADS>());
+  tmem_fence_before_sync();
+  __syncthreads();
+  tmem_fence_after_sync();
+  const unsigned cell = *s_tmem + ((32u * ((unsigned)warp & 3u)) << 16) + (unsigned)(warp >> 2) * 32u;
+#pragma unroll
+  for (int i = 0; i < BlkFft<R>::IPT; ++i)
+#pragma unroll
+    for (int q = 0; q < (R + 3) / 4; ++q) {
+      float2 w[4] = {make_float2(1.f, 0.f), make_float2(1.f, 0.f), make_float2(1.f, 0.f), make_float2(1.f, 0.f)};
+      tw(i, q, w);
+      tmem_st4(cell + TmemTw<R>::at(i, q), w[0], w[1], w[2], w[3]);
+    }
+  tmem_wait_st();
+  return cell;
+}
+// Frees them once every thread is done with its cells.
+template <int THREADS> __device__ __forceinline__ void tmem_release(unsigned base) {
+  tmem_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    tmem_fence_after_sync();
+    tmem_dealloc(base, tmem_cols32<THREADS>());
+  }
+}
+
+// Base of a phase C thread's positions in row r of a column-tiled plane (tiles
+// of 2^lw, lw <= 5); register m is 32 m columns, that is 32 ny m elements, further
+// on.
+__device__ __forceinline__ long long row_pos(int wq, int lane, int r, int ny, int lw) {
+  const int c = wq * 512 + lane;
+  return (((long long)(c >> lw) * ny + r) << lw) + (c & ((1 << lw) - 1));
+}
+
+// Bytes of the forward row pass's shared memory before its stage.
+template <int R, int MODE> __host__ __device__ constexpr size_t rows_fwd_fixed(int nx) {
+  using K = RowB<R, MODE == 1 ? 1 : 3>;
+  return ((size_t)(BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE + (MODE == 1 ? 0 : 3 * K::G * nx)) * 8 +
+          (MODE == 2 ? (size_t)nx * 4 : 0) + 15) / 16 * 16;
+}
+
+// Forward row pass.  MODE 1: scalar RS (one component); 2: VRS (Ex, Ey in;
+// Ex, Ey, Ez out, Ez derived); 3: VRS adjoint (three gradients in and out).
+// Persistent: CTA c handles row groups c, c + grid, ...  Per row group the
+// prologue runs the fused program over every pixel and writes the components
+// to a shared buffer; the stage is then free, so the bulk copies of the next
+// row group start while the component groups transform this one.  Two CTA
+// barriers a row group: after the prologue, and between the phases A and B.  In
+// a scalar row (MODE 1) the thread that needs an element of phase A runs the
+// program for it itself, so there is no buffer and only the second barrier.
+// FK: the fused program's op kinds fixed at compile time (FixedKinds<...>,
+// for the programs the benchmarks and tables run), or FixedKinds<>.
+template <int R, int MODE, class FK = FixedKinds<>>
+__global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, MODE == 1 ? 1 : 3>::MINB)
+    rs_rows_fwd_b(const __grid_constant__ RsLaunch p, const __grid_constant__ RowStage st) {
+  constexpr bool TM = RowB<R, MODE == 1 ? 1 : 3>::TM;
+  __shared__ unsigned s_tmem;
+  constexpr int NC = MODE == 1 ? 1 : 3;
+  constexpr int CIN = MODE;
+  using F = BlkFft<R>;
+  using K = RowB<R, NC>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int nx = p.nx, ny = p.ny;
+  float2* twb = (float2*)smraw;                                      // NTB
+  float2* xch = twb + F::NTB;                                        // LINES x LINE
+  float2* post = xch + K::LINES * F::LINE;                           // NC x G x nx (vector modes)
+  float* xf = (float*)(post + (size_t)NC * K::G * nx);               // nx (VRS: x as float32)
+  const size_t soff = rows_fwd_fixed<R, MODE>(nx);
+  unsigned char* stage = smraw + soff;
+  unsigned long long* mbar = (unsigned long long*)(stage + (size_t)K::G * st.row_bytes);
+  const int tid = threadIdx.x;
+  const int ln = tid / F::T, t = tid % F::T;
+  const int cg = ln / K::G, gi = ln % K::G;
+  const int ngb = (ny + K::G - 1) / K::G;
+  const int total = p.B * ngb;
+  const bool staged = st.n > 0;
+  float2* line = xch + ln * F::LINE;
+  float2* blk = line + (t >> 4) * F::BLK;
+  const bool active = t < F::TB;
+  const GlobalTw<R> twg{blk_tw<R>() + t};
+  typename std::conditional<TM, TmemTw<R>, GlobalTw<R>>::type twa;
+  if constexpr (TM) twa.cell = tmem_twiddles<R, K::THREADS>(&s_tmem, twg);
+  else twa = twg;
+
+  if (tid == 0 && staged) {
+    mbar_init(mbar, 1);
+    fence_mbar_init();
+  }
+  for (int i = tid; i < F::NTB; i += K::THREADS) twb[i] = blk_tw<R>()[F::NTA + i];
+  if constexpr (MODE == 2)
+    for (int i = tid; i < nx; i += K::THREADS) xf[i] = (float)p.x[i];
+  __syncthreads();
+
+  // row groups are taken batch entries fastest: CTAs that run together read the
+  // same rows of the parameter planes a batch shares, which then come from L2
+  auto issue = [&](int grp) {
+    const int b = grp % p.B, r0 = (grp / p.B) * K::G;
+    stage_rows(st, stage, mbar, b, r0, min(K::G, ny - r0));
+  };
+  if (tid == 0 && staged && blockIdx.x < total) issue(blockIdx.x);
+
+  unsigned phase = 0;
+  // the copy may still be in flight: let it land, record the event and leave
+  // without issuing another
+  auto timed_out = [&]() {
+    mbar_wait_bounded(mbar, phase);
+    if (tid == 0) record_timeout();
+    if constexpr (TM) tmem_release<K::THREADS>(s_tmem);
+  };
+  auto next_stage = [&](int grp) {
+    phase ^= 1u;
+    if (tid == 0 && staged && grp + gridDim.x < total) {
+      fence_proxy_async();
+      issue(grp + gridDim.x);
+    }
+  };
+  for (int grp = blockIdx.x; grp < total; grp += gridDim.x) {
+    const int b = grp % p.B;
+    const int r0 = (grp / p.B) * K::G;
+    // a wait that runs out is acted on at the barrier after the prologue
+    // (the prologue then works on stale data, and the launch's output is not
+    // valid), so that no extra barrier is taken per row group
+    const bool got = !staged || mbar_wait_bounded(mbar, phase, g_wait_limit_ns);
+    const int r = r0 + gi;
+    const bool live = r < ny;
+    float2 v[16];
+    if constexpr (MODE == 1) {
+      // this thread's elements, four at a time and then the rest; positions
+      // past the row or the field take a valid pixel and are zeroed
+      const int rr = live ? r : ny - 1;
+      auto chunk = [&](auto npx, auto first) {
+        constexpr int NPX = decltype(npx)::value, F0 = decltype(first)::value, H = R / 2;
+        float2 e[NPX][3];
+        PixelCtx px[NPX];
+        StagedParams pr[NPX];
+#pragma unroll
+        for (int q = 0; q < NPX; ++q) {
+          const int n = min(t + (F0 + q) / H * F::T + 256 * ((F0 + q) % H), nx - 1);
+          const long long pix = (long long)rr * nx + n;
+          const int fo = st.fld[0];
+          e[q][0] = fo >= 0 ? ((const float2*)(stage + fo))[(rr - r0) * nx + n] : p.in[0][(long long)b * p.ibs + pix];
+          e[q][1] = e[q][2] = make_float2(0.f, 0.f);
+          px[q] = PixelCtx{rr, n, pix, b};
+          pr[q] = StagedParams{stage, &st, rr - r0, nx, n};
+        }
+        if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
+        else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
+#pragma unroll
+        for (int q = 0; q < NPX; ++q) {
+          const int f = F0 + q;
+          const bool in = live && t + f / H * F::T + 256 * (f % H) < nx;
+          v[f / H * R + f % H] = in ? e[q][0] : make_float2(0.f, 0.f);
+        }
+      };
+      constexpr int N = F::IPT * R / 2;   // 5 to 8
+      chunk(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{});
+      chunk(std::integral_constant<int, N - 4>{}, std::integral_constant<int, 4>{});
+    } else {
+      const int lim = min(K::G, ny - r0) * nx;
+      const float zb = MODE == 2 ? (float)p.z[b] : 0.f;
+      // one row per group (2304-point lines and longer): its y and y^2 + z^2
+      // once for the group instead of once per pixel
+      const float Y0 = MODE == 2 && K::G == 1 ? (float)p.y[r0] : 0.f;
+      const float z20 = Y0 * Y0 + zb * zb;
+      auto chunk = [&](auto npx, int base) {
+        constexpr int NPX = decltype(npx)::value;
+        float2 e[NPX][3];
+        PixelCtx px[NPX];
+        StagedParams pr[NPX];
+  #pragma unroll
+        for (int q = 0; q < NPX; ++q) {
+          const int idx = base + q * K::THREADS;
+          const int g2 = K::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, r = r0 + g2;
+          const long long pix = (long long)r * nx + n;
+  #pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            e[q][c] = make_float2(0.f, 0.f);
+            if (c < CIN) {
+              const int fo = st.fld[c];
+              e[q][c] = fo >= 0 ? ((const float2*)(stage + fo))[g2 * nx + n] : p.in[c][(long long)b * p.ibs + pix];
+            }
+          }
+          px[q] = PixelCtx{r, n, pix, b};
+          pr[q] = StagedParams{stage, &st, g2, nx, n};
+        }
+        if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
+        else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
+  #pragma unroll
+        for (int q = 0; q < NPX; ++q) {
+          const int r = px[q].row, n = px[q].col;
+          if constexpr (MODE == 2) {  // vectorized_optics.py:258-261, Ez = Ex X/r + Ey Y/r
+            const float Y = K::G == 1 ? Y0 : (float)p.y[r];
+            const float z2 = K::G == 1 ? z20 : Y * Y + zb * zb;
+            const float X = xf[n];
+            const float inv = rsqrtf(X * X + z2);
+            e[q][2] = cadd(cscale(e[q][0], X * inv), cscale(e[q][1], Y * inv));
+          }
+  #pragma unroll
+          for (int c = 0; c < NC; ++c) post[(c * K::G + (r - r0)) * nx + n] = e[q][c];
+        }
+      };
+      {
+        int base = tid;
+        // CTAs of up to 256 threads: four pixels per thread at a time while four
+        // remain, so that their loads and arithmetic overlap and each op of the
+        // program is dispatched once for the four (larger CTAs ran slower so)
+        if constexpr (K::THREADS <= 256)
+          for (; base + 3 * K::THREADS < lim; base += 4 * K::THREADS) chunk(std::integral_constant<int, 4>{}, base);
+        for (; base < lim; base += K::THREADS) chunk(std::integral_constant<int, 1>{}, base);
+      }
+      // every thread has read the stage and written its pixels; every thread
+      // takes the timeout branch or none does
+      if (__syncthreads_or(!got)) return timed_out();
+      next_stage(grp);
+      const float2* src = post + (cg * K::G + gi) * nx;
+#pragma unroll
+      for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+        for (int n1 = 0; n1 < R / 2; ++n1) {
+          const int n = t + i * F::T + 256 * n1;
+          v[i * R + n1] = (live && n < nx) ? src[n] : make_float2(0.f, 0.f);
+        }
+    }
+    blk_a_fwd<R, -1, true>(v, t, line, twa);
+    if constexpr (MODE == 1) {
+      if (__syncthreads_or(!got)) return timed_out();
+      next_stage(grp);
+    } else {
+      __syncthreads();
+    }
+    if (active) {
+      blk_b_fwd<-1>(v, t & 15, blk, twb);
+      __syncwarp();
+      blk_c_fwd<-1>(v, t & 15, blk);
+      if (live) {
+        float2* o = p.work + ((long long)b * NC + cg) * ny * F::P + row_pos(t >> 5, t & 31, r, ny, p.lw);
+        long long step = 32LL * ny;
+        asm volatile("" : "+l"(o), "+l"(step));   // one base, not sixteen addresses live across the loop
+#pragma unroll
+        for (int q = 0; q < 16; ++q) o[q * step] = v[q];
+      }
+    }
+    if constexpr (MODE == 1) __syncthreads();   // the next row's phase A stores to the slots phase C loads here
+  }
+  if constexpr (TM) tmem_release<K::THREADS>(s_tmem);
+}
+
+// Inverse row pass: inverse P-point FFT per row and component, crop to nx
+// columns, optional fused epilogue program (or, for the VRS adjoint, the fold
+// of the Ez gradient into Ex, Ey), store.  Persistent, with the component
+// groups of RowB; each thread's loads of its next row are in flight in
+// registers while the current one is transformed.  With an epilogue phase A
+// leaves the row in its own slots, since the program needs every component of
+// a pixel.
+//
+// What bounds it: the loads in flight, which occupy L1 by whole 128-byte lines
+// (a row's pieces are 64 bytes), so shared memory is kept small: with two sets
+// of lines (one barrier a row instead of two) 8 x 2048^2 VRS took 728 us
+// against 464, and with the phase A twiddles read through L1 instead of kept
+// in Tensor Memory 561; loads that do not allocate in L1 took 628.  Stockham
+// engine: 573.  (16 x 1024^2 scalar, three CTAs an SM: 84 us, 123 on Stockham;
+// with Tensor Memory 95.)
+template <int R, int COUT, bool EPI>
+__global__ void __launch_bounds__(RowB<R, COUT>::THREADS, RowB<R, COUT>::MINB)
+    rs_rows_inv_b(const __grid_constant__ RsLaunch p) {
+  constexpr bool TM = RowB<R, COUT>::TM;
+  __shared__ unsigned s_tmem;
+  using F = BlkFft<R>;
+  using K = RowB<R, COUT>;
+  static_assert(K::CG == COUT, "every component of a row at once");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* twb = (float2*)smraw;
+  float2* line = twb + F::NTB + (threadIdx.x / F::T) * F::LINE;   // LINES x LINE
+  const int tid = threadIdx.x;
+  const int ln = tid / F::T, t = tid % F::T;
+  const int cg = ln / K::G, gi = ln % K::G;
+  const int nx = p.nx, ny = p.ny;
+  const int ngb = (ny + K::G - 1) / K::G;
+  const int total = p.B * ngb;
+  const bool active = t < F::TB;
+  for (int i = tid; i < F::NTB; i += K::THREADS) twb[i] = blk_tw<R>()[F::NTA + i];
+  const GlobalTw<R> twg{blk_tw<R>() + t};
+  typename std::conditional<TM, TmemTw<R>, GlobalTw<R>>::type twa;
+  if constexpr (TM) twa.cell = tmem_twiddles<R, K::THREADS>(&s_tmem, twg);
+  else twa = twg;
+  __syncthreads();
+
+  auto load = [&](int grp, float2 (&d)[16]) {   // row groups batch entries fastest
+    const int b = grp % p.B;
+    int r = (grp / p.B) * K::G + gi;
+    r = r < ny ? r : ny - 1;    // rows past the end load a valid row and discard it
+    const float2* q = p.work + ((long long)b * COUT + cg) * ny * F::P + row_pos(t >> 5, t & 31, r, ny, p.lw);
+    long long step = 32LL * ny;
+    asm volatile("" : "+l"(q), "+l"(step));
+#pragma unroll
+    for (int m = 0; m < 16; ++m) d[m] = q[m * step];
+  };
+
+  float2 nxt[16];
+  if (active && blockIdx.x < total) load(blockIdx.x, nxt);
+  for (int grp = blockIdx.x; grp < total; grp += gridDim.x) {
+    const int b = grp % p.B;
+    const int r0 = (grp / p.B) * K::G;
+    const int r = r0 + gi;
+    float2 v[16];
+    if (active) {
+      float2* blk = line + (t >> 4) * F::BLK;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) v[m] = nxt[m];
+      if (grp + gridDim.x < total) load(grp + gridDim.x, nxt);
+      blk_c_inv<1>(v, t & 15, blk);
+      __syncwarp();
+      blk_b_inv<1>(v, t & 15, blk, twb);
+    }
+    if constexpr (!EPI && K::CG > 1) GroupSync{1 + cg, K::G * F::T}();   // the component groups never meet
+    else __syncthreads();
+    blk_a_inv<R, 1>(v, t, line, twa);
+    if constexpr (!EPI) {
+      if (r < ny) {
+        float2* o = p.out[cg] + (long long)b * p.obs + (long long)r * nx;
+#pragma unroll
+        for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+          for (int n1 = 0; n1 < R / 2; ++n1) {
+            const int n = t + i * F::T + 256 * n1;
+            if (n < nx) o[n] = v[i * R + n1];
+          }
+      }
+    } else {
+      float2* d = line + blk_slot(t);
+#pragma unroll
+      for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+        for (int n1 = 0; n1 < R / 2; ++n1) d[n1 * F::BLK + i * (F::T / 16) * 18] = v[i * R + n1];
+      __syncthreads();
+      const bool fold = p.adjoint && COUT == 3;   // VRS adjoint: Ez gradient folded into Ex, Ey
+      const float zb = fold ? (float)p.z[b] : 0.f;
+      int last = -1;
+      float Y = 0.f, z2 = 0.f;
+      for (int idx = tid; idx < K::G * nx; idx += K::THREADS) {
+        const int g2 = K::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, ro = r0 + g2;
+        if (ro >= ny) break;
+        const long long o = (long long)b * p.obs + (long long)ro * nx + n;
+        const float2* s = twb + F::NTB + g2 * F::LINE + (n >> 8) * F::BLK + blk_slot(n & 255);
+        float2 e[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) e[c] = c < COUT ? s[c * K::G * F::LINE] : make_float2(0.f, 0.f);
+        if (fold) {  // adjoint of Ez = Ex X/r + Ey Y/r (vectorized_optics.py:258-261)
+          if (g2 != last) {
+            last = g2;
+            Y = (float)p.y[ro];
+            z2 = Y * Y + zb * zb;
+          }
+          const float X = (float)p.x[n];
+          const float inv = rsqrtf(X * X + z2);
+          p.out[0][o] = cadd(e[0], cscale(e[2], X * inv));
+          p.out[1][o] = cadd(e[1], cscale(e[2], Y * inv));
+          if (p.out[2]) p.out[2][o] = e[2];   // the unfolded Ez gradient, when asked for
+          continue;
+        }
+        PixelCtx px{ro, n, (long long)ro * nx + n, b};
+        apply_prog(p.post, e, px);
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) p.out[c][o] = e[c];
+      }
+    }
+    // the next row's phase C stores to slots that phase A (or the epilogue) loads here
+    if constexpr (!EPI && K::CG > 1) GroupSync{1 + cg, K::G * F::T}();
+    else __syncthreads();
+  }
+  if constexpr (TM) tmem_release<K::THREADS>(s_tmem);
+}
+
+// ---- transfer spectra ----
+
+// The wrapped offsets (arrays of length 2 Q, Q the power of two the ABI states)
+// rewrapped for px x py points and split into float-float (hi, lo) pairs: offx
+// into off[0 .. px), offy into off[px .. px + py).  `off` is the spectrum
+// buffer, which rs_hhat_cols_b overwrites afterwards.
+static __global__ void rs_split_offsets_b(const double* __restrict__ offx, const double* __restrict__ offy, int q2,
+                                          int px, int py, float2* __restrict__ off) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= px + py) return;
+  const bool isx = i < px;
+  const int n = isx ? px : py, k = isx ? i : i - px;
+  const int d = k < n - k ? k : k - n;                    // index distance
+  const ffloat v = ff_split((isx ? offx : offy)[d < 0 ? d + q2 : d]);
+  off[i] = make_float2(v.hi, v.lo);
+}
+
+// Rows of the wrapped impulse response -> P-point row spectra, row-major in
+// position order.  DZ: the rows of dH/dz instead (the spectrum of the
+// z-derivative).
+template <int R, bool DZ>
+__global__ void __launch_bounds__(RowB<R, 1>::THREADS)
+    rs_hhat_rows_b(int ny, int nx, int py, const float2* __restrict__ off, double zh, const double* __restrict__ zp,
+                   double inv_lambda, float k, float2* __restrict__ out) {
+  using F = BlkFft<R>;
+  using K = RowB<R, 1>;
+  // a distance in device memory, or the host's value
+  const RsGeom g = rs_geom(zp ? __ldg(zp) : zh, inv_lambda, k);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* twb = (float2*)smraw;
+  const int ln = threadIdx.x / F::T, t = threadIdx.x % F::T;
+  float2* line = twb + F::NTB + ln * F::LINE;
+  for (int i = threadIdx.x; i < F::NTB; i += K::THREADS) twb[i] = blk_tw<R>()[F::NTA + i];
+  const int i = blockIdx.x * K::G + ln;   // row of the wrapped response (< py)
+  const bool vy = (i < ny) || (i > py - ny);
+  const float2 oy = off[F::P + i];
+  const ffloat y = {oy.x, oy.y};
+  const ffloat zy = ff_add(g.z2, ff_mul(y, y));
+  float2 v[16];
+#pragma unroll
+  for (int it = 0; it < F::IPT; ++it)
+#pragma unroll
+    for (int n1 = 0; n1 < R; ++n1) {
+      const int col = t + it * F::T + 256 * n1;
+      const bool vx = (col < nx) || (col > F::P - nx);
+      float2 h = make_float2(0.f, 0.f);
+      if (vy && vx) {
+        const float2 ox = off[col];
+        const ffloat x = {ox.x, ox.y};
+        const ffloat sq = ff_add(zy, ff_mul(x, x));
+        h = DZ ? rs_dz_value_s(g, sq) : rs_value_s(g, sq);
+      }
+      v[it * R + n1] = h;
+    }
+  blk_a_fwd<R, -1, false>(v, t, line, GlobalTw<R>{blk_tw<R>() + t});
+  __syncthreads();
+  if (t >= F::TB) return;
+  float2* blk = line + (t >> 4) * F::BLK;
+  blk_b_fwd<-1>(v, t & 15, blk, twb);
+  __syncwarp();
+  blk_c_fwd<-1>(v, t & 15, blk);
+  float2* dst = out + (long long)i * F::P + (t >> 5) * 512 + (t & 31);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) dst[32 * q] = v[q];
+}
+
+// ---- launches ----
 
 template <int R> static int launch_cols_b(cudaStream_t st, const RsLaunch& p) {
   using K = RsColB<R>;
@@ -324,4 +811,87 @@ template <int R> static int launch_hhat_cols_b(cudaStream_t st, const float2* in
   return XL_OK;
 }
 
+template <int R, int MODE, class FK = FixedKinds<>>
+static int launch_rows_fwd_b(cudaStream_t s, const RsLaunch& p) {
+  using K = RowB<R, MODE == 1 ? 1 : 3>;
+  const size_t fixed = rows_fwd_fixed<R, MODE>(p.nx);
+  RowStage st;
+  plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, K::G, fixed, st);
+  const size_t sm = fixed + (size_t)K::G * st.row_bytes + 16;
+  cudaError_t e = allow_smem(rs_rows_fwd_b<R, MODE, FK>, sm);
+  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_fwd_b smem");
+  const int total = p.B * ((p.ny + K::G - 1) / K::G);
+  const int grid = persistent_grid(rs_rows_fwd_b<R, MODE, FK>, K::THREADS, sm, total);
+  rs_rows_fwd_b<R, MODE, FK><<<grid, K::THREADS, sm, s>>>(p, st);
+  XL_CHECK_LAUNCH("rs_rows_fwd_b");
+  return XL_OK;
+}
+
+template <int R, int COUT, bool EPI> static int launch_rows_inv_b(cudaStream_t s, const RsLaunch& p) {
+  using K = RowB<R, COUT>;
+  const size_t sm = ((size_t)BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE) * 8;
+  cudaError_t e = allow_smem(rs_rows_inv_b<R, COUT, EPI>, sm);
+  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_inv_b smem");
+  const int total = p.B * ((p.ny + K::G - 1) / K::G);
+  const int grid = persistent_grid(rs_rows_inv_b<R, COUT, EPI>, K::THREADS, sm, total);
+  rs_rows_inv_b<R, COUT, EPI><<<grid, K::THREADS, sm, s>>>(p);
+  XL_CHECK_LAUNCH("rs_rows_inv_b");
+  return XL_OK;
+}
+
+template <int R> int rs_blk_rows(cudaStream_t st, const RsLaunch& p, bool inverse) {
+  if (!inverse) {
+    // the programs of the benchmarks' fields get a kernel with their op kinds
+    // fixed: a phase SLM before scalar RS, an LCD and a polarizer before VRS
+    using SlmOnly = FixedKinds<XL_OP_PHASE>;
+    using LcdLp = FixedKinds<XL_OP_LCD, XL_OP_LP>;
+    if (p.cout == 1) {
+      if constexpr (R >= 8)
+        if (SlmOnly::matches(p.pre)) return launch_rows_fwd_b<R, 1, SlmOnly>(st, p);
+      return launch_rows_fwd_b<R, 1>(st, p);
+    }
+    if (p.cin == 2) {
+      if constexpr (R >= 8)
+        if (LcdLp::matches(p.pre)) return launch_rows_fwd_b<R, 2, LcdLp>(st, p);
+      return launch_rows_fwd_b<R, 2>(st, p);
+    }
+    return launch_rows_fwd_b<R, 3>(st, p);
+  }
+  const bool epi = p.post.nops > 0 || (p.adjoint && p.cout == 3);
+  if (p.cout == 1) return epi ? launch_rows_inv_b<R, 1, true>(st, p) : launch_rows_inv_b<R, 1, false>(st, p);
+  return epi ? launch_rows_inv_b<R, 3, true>(st, p) : launch_rows_inv_b<R, 3, false>(st, p);
+}
+
+template <int R> int rs_blk_cols(cudaStream_t st, const RsLaunch& p) { return launch_cols_b<R>(st, p); }
+
+template <int R>
+int rs_blk_hhat_rows(cudaStream_t st, int ny, int nx, int py, const double* offx, const double* offy, int q2, double z,
+                     const double* zp, double wavelength, int dz, float2* off, float2* out) {
+  using F = BlkFft<R>;
+  using K = RowB<R, 1>;
+  rs_split_offsets_b<<<(F::P + py + 255) / 256, 256, 0, st>>>(offx, offy, q2, F::P, py, off);
+  XL_CHECK_LAUNCH("rs_split_offsets_b");
+  const size_t sm = ((size_t)F::NTB + K::LINES * F::LINE) * 8;
+  const float k = (float)(2.0 * M_PI / wavelength);
+  auto run = [&](auto kernel) {
+    cudaError_t e = allow_smem(kernel, sm);
+    if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_rows_b smem");
+    kernel<<<py / K::G, K::THREADS, sm, st>>>(ny, nx, py, off, z, zp, 1.0 / wavelength, k, out);
+    XL_CHECK_LAUNCH("rs_hhat_rows_b");
+    return (int)XL_OK;
+  };
+  return dz ? run(rs_hhat_rows_b<R, true>) : run(rs_hhat_rows_b<R, false>);
+}
+
+template <int R> int rs_blk_hhat_cols(cudaStream_t st, const float2* in, int px, float scale, float2* out) {
+  return launch_hhat_cols_b<R>(st, in, px, scale, out);
+}
+
 }  // namespace xl
+
+#define XL_RS_BLK_INSTANTIATE(R)                                                                             \
+  template int xl::rs_blk_rows<R>(cudaStream_t, const RsLaunch&, bool);                                      \
+  template int xl::rs_blk_cols<R>(cudaStream_t, const RsLaunch&);                                            \
+  template int xl::rs_blk_hhat_rows<R>(cudaStream_t, int, int, int, const double*, const double*, int, double, \
+                                       const double*, double, int, float2*, float2*);                        \
+  template int xl::rs_blk_hhat_cols<R>(cudaStream_t, const float2*, int, float, float2*);

@@ -24,8 +24,8 @@ struct RsLaunch {
   float2* work;
   XlProg pre, post;
   int adjoint;
-  int px;                       // columns of the intermediate (the x transform's length)
-  int lw;                       // log2 of its column-tile width
+  int px, py;                   // points of the x and the y transform (px: columns of the intermediate)
+  int lw;                       // log2 of the intermediate's column-tile width (block engine)
 };
 
 // Q = 2^logq is the half transform length: the smallest power of two >= the field side.
@@ -37,8 +37,34 @@ inline int rs_logq(int ny, int nx) {
   return l < 5 ? 5 : l;
 }
 
+// Fields whose longer side is 257 to 2048 run on the block FFT engine, each
+// axis with its own transform length P = 256 R, the shortest the engine has
+// (R = 4, 6, .. 16) that holds the axis's 2 n - 1 points of linear
+// convolution.  Shorter and longer ones run both axes at 2 Q points on the
+// Stockham engine.
+inline bool rs_is_blk(int ny, int nx) {
+  const int n = ny > nx ? ny : nx;
+  return n > 256 && n <= 2048;
+}
+inline int rs_blk_r(int n) {
+  return n <= 512 ? 4 : (n <= 1024 ? 8 : 16);
+}
+// Points of the x (or y) transform of an ny x nx field.
+inline int rs_px(int ny, int nx) { return rs_is_blk(ny, nx) ? 256 * rs_blk_r(nx) : 2 << rs_logq(ny, nx); }
+inline int rs_py(int ny, int nx) { return rs_is_blk(ny, nx) ? 256 * rs_blk_r(ny) : 2 << rs_logq(ny, nx); }
+
+// Block engine passes (explicitly instantiated for R = 4, 6, .. 16 in the
+// kernel translation units rs_b*.cu).  hhat_rows: offx / offy wrapped for q2
+// points, split into `off` (px + py entries) on the way.
+template <int R> int rs_blk_rows(cudaStream_t st, const RsLaunch& p, bool inverse);
+template <int R> int rs_blk_cols(cudaStream_t st, const RsLaunch& p);
+template <int R>
+int rs_blk_hhat_rows(cudaStream_t st, int ny, int nx, int py, const double* offx, const double* offy, int q2, double z,
+                     const double* zp, double wavelength, int dz, float2* off, float2* out);
+template <int R> int rs_blk_hhat_cols(cudaStream_t st, const float2* in, int px, float scale, float2* out);
+
 // Transfer spectrum and propagation passes for Q = 2^LOGQ (explicitly
-// instantiated for LOGQ = 4..12 in the kernel translation units).
+// instantiated for LOGQ = 5..8 and 12 in the kernel translation units).
 template <int LOGQ>
 int rs_spectrum(cudaStream_t st, int ny, int nx, const double* offx, const double* offy, double z,
                 const double* zp, double wavelength, double scale, float2* spec, float2* work, int dz);

@@ -36,7 +36,6 @@
 #include <vector>
 
 #include "line_fft.cuh"
-#include "rs_blk.cuh"
 #include "rs_host.h"
 
 namespace xl {
@@ -57,10 +56,10 @@ template <int LOGQ> struct RsCfg {
   // Column-tile width of the intermediate and spectrum layouts.  At Q = 2048
   // the tiles are 8 columns wide, so a warp's row access is four 64-byte
   // pieces; the column pass takes half a tile per CTA.
-  static constexpr int W = LOGQ >= 12 ? 2 : (LOGQ == 11 ? 8 : ((32 / T) > 4 ? (32 / T) : 4));
+  static constexpr int W = LOGQ >= 12 ? 2 : ((32 / T) > 4 ? (32 / T) : 4);
   // Column-pass (and spectrum-build) CTAs take CW columns of a tile,
   // interleaved in the lanes of every warp.
-  static constexpr int CW = LOGQ == 11 ? 4 : W;
+  static constexpr int CW = W;
   // the transfer spectrum is tiled CW wide: exactly the columns of one
   // column-pass CTA, so its reads are whole 32-byte pieces
   static constexpr int SW = CW;
@@ -551,15 +550,11 @@ int rs_spectrum(cudaStream_t st, int ny, int nx, const double* offx, const doubl
                                                                            k, work);
   }
   XL_CHECK_LAUNCH("rs_hhat_rows");
-  if constexpr (LOGQ >= 9 && LOGQ <= 11) {
-    return launch_hhat_cols_b<C::P / 256>(st, work, C::P, (float)scale, spec);
-  } else {
-    const size_t sm2 = (size_t)C::CW * C::CXS * sizeof(float2);
-    e = allow_smem(rs_hhat_cols<LOGQ>, sm2);
-    if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols smem");
-    rs_hhat_cols<LOGQ><<<C::P / C::CW, C::COL_THREADS, sm2, st>>>(work, (float)scale, spec);
-    XL_CHECK_LAUNCH("rs_hhat_cols");
-  }
+  const size_t sm2 = (size_t)C::CW * C::CXS * sizeof(float2);
+  e = allow_smem(rs_hhat_cols<LOGQ>, sm2);
+  if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols smem");
+  rs_hhat_cols<LOGQ><<<C::P / C::CW, C::COL_THREADS, sm2, st>>>(work, (float)scale, spec);
+  XL_CHECK_LAUNCH("rs_hhat_cols");
   return XL_OK;
 }
 
@@ -636,8 +631,7 @@ static int launch_stage(cudaStream_t st, const RsLaunch& p, int stage) {
     }
     return launch_rows_fwd<LOGQ, 3>(st, p);
   } else if (stage == 1) {
-    if constexpr (LOGQ >= 9 && LOGQ <= 11) return launch_cols_b<C::P / 256>(st, p);
-    else return launch_cols<LOGQ>(st, p);
+    return launch_cols<LOGQ>(st, p);
   } else {
     const bool epi = p.post.nops > 0 || (p.adjoint && p.cout == 3);
     if (p.cout == 1) return epi ? launch_rows_inv<LOGQ, 1, true>(st, p) : launch_rows_inv<LOGQ, 1, false>(st, p);
@@ -647,10 +641,7 @@ static int launch_stage(cudaStream_t st, const RsLaunch& p, int stage) {
 }
 
 template <int LOGQ>
-int rs_propagate(cudaStream_t st, const RsLaunch& q, int stage) {
-  RsLaunch p = q;
-  p.px = RsCfg<LOGQ>::P;
-  p.lw = RsCfg<LOGQ>::W == 8 ? 3 : (RsCfg<LOGQ>::W == 4 ? 2 : 1);
+int rs_propagate(cudaStream_t st, const RsLaunch& p, int stage) {
   if (stage >= 0) return launch_stage<LOGQ>(st, p, stage);
   for (int s = 0; s < 3; ++s)
     if (int rc = launch_stage<LOGQ>(st, p, s)) return rc;

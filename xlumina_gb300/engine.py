@@ -533,8 +533,9 @@ def build_rs_spectrum(x, y, z, wavelength, dz=False) -> torch.Tensor:
     dev = device()
     offx = device_array(rs_wrapped_offsets(x, P), torch.float64)
     offy = device_array(rs_wrapped_offsets(y, P), torch.float64)
-    spec = torch.empty(P * P, dtype=torch.complex64, device=dev)
-    work = torch.empty(P * P, dtype=torch.complex64, device=dev)
+    size = L.xl_rs_spectrum_bytes(ny, nx) // 8
+    spec = torch.empty(size, dtype=torch.complex64, device=dev)
+    work = torch.empty(L.xl_rs_spectrum_work_bytes(ny, nx) // 8, dtype=torch.complex64, device=dev)
     dx = x[1] - x[0]
     dy = y[1] - y[0]
     scale = dx * dy / float(P * P)
@@ -579,12 +580,13 @@ def build_rs_spectra_device(x, y, zd: torch.Tensor, wavelength, dz=False) -> tor
     offx = device_offsets(x, P)
     offy = device_offsets(y, P)
     n = zd.numel()
-    spec = torch.empty((n, P * P), dtype=torch.complex64, device=dev)
-    work = torch.empty(P * P, dtype=torch.complex64, device=dev)
+    size = L.xl_rs_spectrum_bytes(ny, nx) // 8
+    spec = torch.empty((n, size), dtype=torch.complex64, device=dev)
+    work = torch.empty(L.xl_rs_spectrum_work_bytes(ny, nx) // 8, dtype=torch.complex64, device=dev)
     scale = (x[1] - x[0]) * (y[1] - y[0]) / float(P * P)
     _lib.check(L.xl_rs_transfer_spectra_device_z(stream_handle(), ny, nx, offx.data_ptr(), offy.data_ptr(),
                                                  zd.data_ptr(), n, float(wavelength), scale, 1 if dz else 0,
-                                                 spec.data_ptr(), P * P, work.data_ptr()),
+                                                 spec.data_ptr(), size, work.data_ptr()),
                "xl_rs_transfer_spectra_device_z")
     return spec
 
