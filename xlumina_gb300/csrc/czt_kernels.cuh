@@ -359,10 +359,10 @@ static int launch_czt_rows(cudaStream_t s, const CztLaunch& p) {
     set_error("czt: input row of %d columns too long for shared memory", p.nx);
     return XL_EUNSUPPORTED;
   }
-  cudaError_t e = allow_smem(czt_rows<LOGL, NC, ZU, MB, FK, OG>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "czt_rows smem");
+  int per_sm;
+  if (int rc = launch_ready<czt_rows<LOGL, NC, ZU, MB, FK, OG>>(F::THREADS, sm, &per_sm, "czt_rows")) return rc;
   const int total = p.B * ((p.ny + C::G - 1) / C::G);
-  const int grid = persistent_grid(czt_rows<LOGL, NC, ZU, MB, FK, OG>, F::THREADS, sm, total);
+  const int grid = persistent_grid(per_sm, total);
   czt_rows<LOGL, NC, ZU, MB, FK, OG><<<grid, F::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("czt_rows");
   return XL_OK;
@@ -398,14 +398,13 @@ static int launch_czt_cols(cudaStream_t s, const CztLaunch& p) {
   const size_t sm = (size_t)(C::W * C::CXS + C::NTW) * sizeof(float2);
   // kernel variant: 0 one CTA per column tile and entry; 1 persistent
   if (kernel_variant(XL_PASS_CZT_COLS, LOGL) == 1) {
-    cudaError_t e = allow_smem(czt_cols<LOGL, ZU, true>, sm);
-    if (e != cudaSuccess) return cuda_fail(e, "czt_cols smem");
-    const int grid = persistent_grid(czt_cols<LOGL, ZU, true>, C::COL_THREADS, sm,
-                                     ((p.mx + C::W - 1) / C::W) * p.B);
+    int per_sm;
+    if (int rc = launch_ready<czt_cols<LOGL, ZU, true>>(C::COL_THREADS, sm, &per_sm, "czt_cols")) return rc;
+    const int grid = persistent_grid(per_sm, ((p.mx + C::W - 1) / C::W) * p.B);
     czt_cols<LOGL, ZU, true><<<grid, C::COL_THREADS, sm, s>>>(p);
   } else {
-    cudaError_t e = allow_smem(czt_cols<LOGL, ZU>, sm);
-    if (e != cudaSuccess) return cuda_fail(e, "czt_cols smem");
+    int per_sm;
+    if (int rc = launch_ready<czt_cols<LOGL, ZU>>(C::COL_THREADS, sm, &per_sm, "czt_cols")) return rc;
     czt_cols<LOGL, ZU><<<dim3((p.mx + C::W - 1) / C::W, p.B), C::COL_THREADS, sm, s>>>(p);
   }
   XL_CHECK_LAUNCH("czt_cols");

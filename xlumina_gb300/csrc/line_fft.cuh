@@ -11,6 +11,7 @@
 
 #include <stdint.h>
 
+#include <atomic>
 #include <vector>
 
 #include "common.cuh"
@@ -184,13 +185,43 @@ static inline int device_sms() {
   return sms[dev];
 }
 
+// Launch preparation of a kernel, once per device instead of once per launch:
+// the dynamic shared memory limit raised to what the device allows, and the
+// resident CTAs per SM for the last shared memory size asked for.
+template <auto KERNEL>
+static int launch_ready(int threads, size_t smem, int* per_sm, const char* what) {
+  static std::atomic<unsigned long long> cache[64];   // (smem << 8 | CTAs per SM), 0: not prepared
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e, what);
+  std::atomic<unsigned long long>* slot = dev >= 0 && dev < 64 ? &cache[dev] : nullptr;
+  const unsigned long long have = slot ? slot->load(std::memory_order_acquire) : 0;
+  if (have && (have >> 8) == smem) {
+    *per_sm = (int)(have & 255);
+    return XL_OK;
+  }
+  if (!have) {
+    cudaFuncAttributes at;
+    if ((e = cudaFuncGetAttributes(&at, KERNEL)) != cudaSuccess) return cuda_fail(e, what);
+    int most = 0;
+    if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
+      return cuda_fail(e, what);
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    if (e != cudaSuccess) return cuda_fail(e, what);
+  }
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, threads, smem) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = 1;
+  }
+  if (n > 255) n = 255;
+  if (slot) slot->store((unsigned long long)smem << 8 | (unsigned)n, std::memory_order_release);
+  *per_sm = n;
+  return XL_OK;
+}
+
 // Grid of a persistent kernel: every resident CTA slot, at most `work` CTAs.
-template <typename K>
-static int persistent_grid(K kernel, int threads, size_t smem, int work) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
+static inline int persistent_grid(int per_sm, long long work) {
   const long long g = (long long)per_sm * device_sms();
   return (int)(g < work ? g : work);
 }

@@ -794,9 +794,9 @@ __global__ void __launch_bounds__(RowB<R, 1>::THREADS)
 
 template <int R> static int launch_cols_b(cudaStream_t st, const RsLaunch& p) {
   using K = RsColB<R>;
-  cudaError_t e = allow_smem(rs_cols_b<R>, K::SMEM);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_cols_b smem");
-  const int grid = persistent_grid(rs_cols_b<R>, K::THREADS, K::SMEM, p.B * (p.px / K::CW));
+  int per_sm;
+  if (int rc = launch_ready<rs_cols_b<R>>(K::THREADS, K::SMEM, &per_sm, "rs_cols_b")) return rc;
+  const int grid = persistent_grid(per_sm, p.B * (p.px / K::CW));
   rs_cols_b<R><<<grid, K::THREADS, K::SMEM, st>>>(p);
   XL_CHECK_LAUNCH("rs_cols_b");
   return XL_OK;
@@ -804,8 +804,8 @@ template <int R> static int launch_cols_b(cudaStream_t st, const RsLaunch& p) {
 
 template <int R> static int launch_hhat_cols_b(cudaStream_t st, const float2* in, int px, float scale, float2* out) {
   using K = RsColB<R>;
-  cudaError_t e = allow_smem(rs_hhat_cols_b<R>, K::SMEM);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols_b smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_hhat_cols_b<R>>(K::THREADS, K::SMEM, &per_sm, "rs_hhat_cols_b")) return rc;
   rs_hhat_cols_b<R><<<px / K::CW, K::THREADS, K::SMEM, st>>>(in, px, scale, out);
   XL_CHECK_LAUNCH("rs_hhat_cols_b");
   return XL_OK;
@@ -818,10 +818,10 @@ static int launch_rows_fwd_b(cudaStream_t s, const RsLaunch& p) {
   RowStage st;
   plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, K::G, fixed, st);
   const size_t sm = fixed + (size_t)K::G * st.row_bytes + 16;
-  cudaError_t e = allow_smem(rs_rows_fwd_b<R, MODE, FK>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_fwd_b smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_rows_fwd_b<R, MODE, FK>>(K::THREADS, sm, &per_sm, "rs_rows_fwd_b")) return rc;
   const int total = p.B * ((p.ny + K::G - 1) / K::G);
-  const int grid = persistent_grid(rs_rows_fwd_b<R, MODE, FK>, K::THREADS, sm, total);
+  const int grid = persistent_grid(per_sm, total);
   rs_rows_fwd_b<R, MODE, FK><<<grid, K::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("rs_rows_fwd_b");
   return XL_OK;
@@ -830,10 +830,10 @@ static int launch_rows_fwd_b(cudaStream_t s, const RsLaunch& p) {
 template <int R, int COUT, bool EPI> static int launch_rows_inv_b(cudaStream_t s, const RsLaunch& p) {
   using K = RowB<R, COUT>;
   const size_t sm = ((size_t)BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE) * 8;
-  cudaError_t e = allow_smem(rs_rows_inv_b<R, COUT, EPI>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_inv_b smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_rows_inv_b<R, COUT, EPI>>(K::THREADS, sm, &per_sm, "rs_rows_inv_b")) return rc;
   const int total = p.B * ((p.ny + K::G - 1) / K::G);
-  const int grid = persistent_grid(rs_rows_inv_b<R, COUT, EPI>, K::THREADS, sm, total);
+  const int grid = persistent_grid(per_sm, total);
   rs_rows_inv_b<R, COUT, EPI><<<grid, K::THREADS, sm, s>>>(p);
   XL_CHECK_LAUNCH("rs_rows_inv_b");
   return XL_OK;
@@ -873,14 +873,15 @@ int rs_blk_hhat_rows(cudaStream_t st, int ny, int nx, int py, const double* offx
   XL_CHECK_LAUNCH("rs_split_offsets_b");
   const size_t sm = ((size_t)F::NTB + K::LINES * F::LINE) * 8;
   const float k = (float)(2.0 * M_PI / wavelength);
-  auto run = [&](auto kernel) {
-    cudaError_t e = allow_smem(kernel, sm);
-    if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_rows_b smem");
+  int per_sm;
+  auto run = [&](auto kernel, int rc) {
+    if (rc) return rc;
     kernel<<<py / K::G, K::THREADS, sm, st>>>(ny, nx, py, off, z, zp, 1.0 / wavelength, k, out);
     XL_CHECK_LAUNCH("rs_hhat_rows_b");
     return (int)XL_OK;
   };
-  return dz ? run(rs_hhat_rows_b<R, true>) : run(rs_hhat_rows_b<R, false>);
+  if (dz) return run(rs_hhat_rows_b<R, true>, launch_ready<rs_hhat_rows_b<R, true>>(K::THREADS, sm, &per_sm, "rs_hhat_rows_b"));
+  return run(rs_hhat_rows_b<R, false>, launch_ready<rs_hhat_rows_b<R, false>>(K::THREADS, sm, &per_sm, "rs_hhat_rows_b"));
 }
 
 template <int R> int rs_blk_hhat_cols(cudaStream_t st, const float2* in, int px, float scale, float2* out) {

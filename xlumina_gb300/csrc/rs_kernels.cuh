@@ -537,22 +537,21 @@ int rs_spectrum(cudaStream_t st, int ny, int nx, const double* offx, const doubl
   using C = RsCfg<LOGQ>;
   const size_t sm1 = (size_t)C::G * C::XS * sizeof(float2);
   const float k = (float)(2.0 * M_PI / wavelength);
-  cudaError_t e;
+  int per_sm;
   rs_split_offsets<<<(2 * C::P + 255) / 256, 256, 0, st>>>(offx, offy, C::P, spec);
   XL_CHECK_LAUNCH("rs_split_offsets");
   if (dz) {
-    if ((e = allow_smem(rs_hhat_rows<LOGQ, true>, sm1)) != cudaSuccess) return cuda_fail(e, "rs_hhat_rows smem");
+    if (int rc = launch_ready<rs_hhat_rows<LOGQ, true>>(C::ROW_THREADS, sm1, &per_sm, "rs_hhat_rows")) return rc;
     rs_hhat_rows<LOGQ, true><<<C::P / C::G, C::ROW_THREADS, sm1, st>>>(ny, nx, spec, z, zp, 1.0 / wavelength,
                                                                           k, work);
   } else {
-    if ((e = allow_smem(rs_hhat_rows<LOGQ, false>, sm1)) != cudaSuccess) return cuda_fail(e, "rs_hhat_rows smem");
+    if (int rc = launch_ready<rs_hhat_rows<LOGQ, false>>(C::ROW_THREADS, sm1, &per_sm, "rs_hhat_rows")) return rc;
     rs_hhat_rows<LOGQ, false><<<C::P / C::G, C::ROW_THREADS, sm1, st>>>(ny, nx, spec, z, zp, 1.0 / wavelength,
                                                                            k, work);
   }
   XL_CHECK_LAUNCH("rs_hhat_rows");
   const size_t sm2 = (size_t)C::CW * C::CXS * sizeof(float2);
-  e = allow_smem(rs_hhat_cols<LOGQ>, sm2);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_hhat_cols smem");
+  if (int rc = launch_ready<rs_hhat_cols<LOGQ>>(C::COL_THREADS, sm2, &per_sm, "rs_hhat_cols")) return rc;
   rs_hhat_cols<LOGQ><<<C::P / C::CW, C::COL_THREADS, sm2, st>>>(work, (float)scale, spec);
   XL_CHECK_LAUNCH("rs_hhat_cols");
   return XL_OK;
@@ -572,10 +571,10 @@ static int launch_rows_fwd(cudaStream_t s, const RsLaunch& p) {
     set_error("rs: row of %d columns too long for shared memory", p.nx);
     return XL_EUNSUPPORTED;
   }
-  cudaError_t e = allow_smem(rs_rows_fwd<LOGQ, MODE, FK>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_fwd smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_rows_fwd<LOGQ, MODE, FK>>(F::THREADS, sm, &per_sm, "rs_rows_fwd")) return rc;
   const int total = p.B * ((p.ny + C::G - 1) / C::G);
-  const int grid = persistent_grid(rs_rows_fwd<LOGQ, MODE, FK>, F::THREADS, sm, total);
+  const int grid = persistent_grid(per_sm, total);
   rs_rows_fwd<LOGQ, MODE, FK><<<grid, F::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("rs_rows_fwd");
   return XL_OK;
@@ -590,10 +589,10 @@ static int launch_rows_inv(cudaStream_t s, const RsLaunch& p) {
     set_error("rs: row of %d columns too long for shared memory", p.nx);
     return XL_EUNSUPPORTED;
   }
-  cudaError_t e = allow_smem(rs_rows_inv<LOGQ, COUT, EPI>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_rows_inv smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_rows_inv<LOGQ, COUT, EPI>>(F::THREADS, sm, &per_sm, "rs_rows_inv")) return rc;
   const int total = p.B * ((p.ny + C::G - 1) / C::G);
-  const int grid = persistent_grid(rs_rows_inv<LOGQ, COUT, EPI>, F::THREADS, sm, total);
+  const int grid = persistent_grid(per_sm, total);
   rs_rows_inv<LOGQ, COUT, EPI><<<grid, F::THREADS, sm, s>>>(p);
   XL_CHECK_LAUNCH("rs_rows_inv");
   return XL_OK;
@@ -603,8 +602,8 @@ template <int LOGQ>
 static int launch_cols(cudaStream_t st, const RsLaunch& p) {
   using C = RsCfg<LOGQ>;
   const size_t sm = (size_t)(C::CW * C::CXS + C::NTW) * sizeof(float2);
-  cudaError_t e = allow_smem(rs_cols_conv<LOGQ>, sm);
-  if (e != cudaSuccess) return cuda_fail(e, "rs_cols_conv smem");
+  int per_sm;
+  if (int rc = launch_ready<rs_cols_conv<LOGQ>>(C::COL_THREADS, sm, &per_sm, "rs_cols_conv")) return rc;
   rs_cols_conv<LOGQ><<<dim3(p.B, C::P / C::CW), C::COL_THREADS, sm, st>>>(p);
   XL_CHECK_LAUNCH("rs_cols_conv");
   return XL_OK;
