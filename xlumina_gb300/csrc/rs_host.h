@@ -47,7 +47,8 @@ inline bool rs_is_blk(int ny, int nx) {
   return n > 256 && n <= 2048;
 }
 inline int rs_blk_r(int n) {
-  return n <= 512 ? 4 : (n <= 1024 ? 8 : 16);
+  const int r = (2 * n + 511) / 512 * 2;
+  return r < 4 ? 4 : r;
 }
 // Points of the x (or y) transform of an ny x nx field.
 inline int rs_px(int ny, int nx) { return rs_is_blk(ny, nx) ? 256 * rs_blk_r(nx) : 2 << rs_logq(ny, nx); }
