@@ -133,17 +133,14 @@ enum {
   XL_NUM_PASSES = 4
 };
 /* Variants available for `pass` at transform length 2^log2_len (>= 1; 0 if
- * the pass or length is unknown).  Variant 0 is the default kernel shape
- * except at 4096 points: the chirp-z x transform defaults to variant 3
- * (registers sized for two CTAs per SM), the chirp-z y transform to variant
- * 1 (persistent) and the RS column pass to number 8.  The others are the
- * alternatives the autotuner measures against the default.  RS column pass:
- * every number selects the one kernel of that length (the numbers of kernels
- * that earlier releases had are still accepted).  Chirp-z x
- * transform: 0 the stage capped for two CTAs per SM, 1 for one, 2 no
- * stage, 3 as 0 with registers for two CTAs, 4 (4096 points, three
- * components) one component group, two CTAs per SM.  Chirp-z y transform:
- * 0 one CTA per column tile and entry, 1 persistent. */
+ * the pass or length is unknown).  The RS column pass and, at 1024 to 4096
+ * points, the chirp-z transforms have one kernel per length, which every number
+ * selects (the numbers of kernels that earlier releases had are still
+ * accepted; the defaults at 4096 points are 8, 3 and 1).  At the other lengths
+ * variant 0 is the default and the others are the alternatives the autotuner
+ * measures against it.  Chirp-z x transform: 0 the stage capped for two CTAs
+ * per SM, 1 for one, 2 no stage, 3 as 0 with registers for two CTAs.  Chirp-z
+ * y transform: 0 one CTA per column tile and entry, 1 persistent. */
 int xl_kernel_variant_count(int pass, int log2_len);
 /* Select variant `variant` (< the count) for later launches. */
 int xl_set_kernel_variant(int pass, int log2_len, int variant);
@@ -271,7 +268,9 @@ typedef struct {
   int batch, comps_in, comps_out, mode;
   int ny, nx;            /* input plane */
   int my, mx;            /* output plane */
-  int log2_lx, log2_ly;  /* Bluestein lengths (>= nx + mx, >= ny + my) */
+  int log2_lx, log2_ly;  /* Bluestein lengths (>= nx + mx, >= ny + my): log2 of a power of two (5..13),
+                            or (one distance per call) the length itself, 512 k for k = 2..8, with
+                            the spectrum g of that axis in block order (below) */
   const void* in[3];
   long long in_bstride;
   void* out[3];
@@ -284,7 +283,9 @@ typedef struct {
   double cte_re, cte_im; /* constant output factor */
   /* complex64 chirp data per axis (wave_optics.py:385-460, float64 on the host):
    * pre[n] = A^-n h[m-1+n] (m values); g = fft(1/h[:m+M], L) in natural
-   * order; post[l] = h[m-1+l] e^{-i 2 pi l_f (1/2 - m/2)/Dm} / L */
+   * order; post[l] = h[m-1+l] e^{-i 2 pi l_f (1/2 - m/2)/Dm} / L.  Block order
+   * of a length L = 256 R: entry m 16 R + 16 k1 + k2 holds the natural entry
+   * k1 + R (k2 + 16 m), k1 < R, k2 and m < 16. */
   const void* pre_x;
   const void* g_x;
   const void* post_x;

@@ -135,12 +135,12 @@ int read_status(unsigned int* flag, int clear) {
 // 4096 points).  Earlier releases had 9 kernels at 1024 and 2048 points and 11
 // at 4096 (packed two-line, prefetching, barrier groups, radix 64); all were
 // slower than it and are gone, but their numbers are still taken and select
-// it, so that a stored choice keeps working.  The chirp-z x transform: the
-// stage capped for two CTAs per SM (0), every plane staged that fits one CTA
-// per SM (1), no staging (2), as 0 with registers for two CTAs per SM (3),
-// and at 4096 points for three components one group transforming them one
-// after the other, two CTAs per SM (4).  The chirp-z y transform: one CTA per
-// column tile and entry (0), persistent (1).
+// it, so that a stored choice keeps working.  So do
+// the numbers of the chirp-z transforms at those lengths.  At the others, the
+// chirp-z x transform: the stage capped for two CTAs per SM (0), every plane
+// staged that fits one CTA per SM (1), no staging (2), as 0 with registers for
+// two CTAs per SM (3); the chirp-z y transform: one CTA per column tile and
+// entry (0), persistent (1).
 static int variant_count(int pass, int log2_len) {
   if (pass < 0 || pass >= XL_NUM_PASSES || log2_len < 1 || log2_len > 13) return 0;
   if (pass == XL_PASS_RS_COLS && log2_len == 12) return 11;
@@ -152,13 +152,7 @@ static int variant_count(int pass, int log2_len) {
 }
 static std::atomic<int> g_variant[XL_NUM_PASSES][14];
 
-// Defaults that differ from variant 0, by measurement: the 4096-point chirp-z
-// x transform (the 2048^2 high-NA focus) with registers for two CTAs per SM,
-// 1451 against 1400 tables/s on the high-NA optimisation step; the persistent
-// chirp-z y transform at 4096 points: 1945 against 1925 tables/s on the
-// high-NA step (on the 4f step's 2048- and 1024-point transforms it measured
-// 0.3 % slower, so variant 0 stays there).  The RS column pass's 8 is the
-// number its persistent kernel has had.
+// Defaults other than 0: the numbers that the kernels of these lengths have had.
 static const bool g_variant_defaults = [] {
   g_variant[XL_PASS_CZT_ROWS][12].store(3, std::memory_order_relaxed);
   g_variant[XL_PASS_RS_COLS][12].store(8, std::memory_order_relaxed);

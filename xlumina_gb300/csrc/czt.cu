@@ -18,22 +18,45 @@ namespace xl {
     case 7: return FN<7>(__VA_ARGS__);        \
     case 8: return FN<8>(__VA_ARGS__);        \
     case 9: return FN<9>(__VA_ARGS__);        \
-    case 10: return FN<10>(__VA_ARGS__);      \
-    case 11: return FN<11>(__VA_ARGS__);      \
-    case 12: return FN<12>(__VA_ARGS__);      \
     case 13: return FN<13>(__VA_ARGS__);      \
     default: break;                           \
   }
 
-static int dispatch_rows(cudaStream_t st, const CztLaunch& p, int ll) {
+#define XL_CZT_BLK_DISPATCH(LEN, FN, ...)     \
+  switch ((LEN) / 256) {                      \
+    case 4: return FN<4>(__VA_ARGS__);        \
+    case 6: return FN<6>(__VA_ARGS__);        \
+    case 8: return FN<8>(__VA_ARGS__);        \
+    case 10: return FN<10>(__VA_ARGS__);      \
+    case 12: return FN<12>(__VA_ARGS__);      \
+    case 14: return FN<14>(__VA_ARGS__);      \
+    case 16: return FN<16>(__VA_ARGS__);      \
+    default: break;                           \
+  }
+
+// A Bluestein length as XlCztArgs gives it: its log2, or itself.  0: neither.
+static int czt_len(int v) {
+  if (v >= 5 && v <= 13) return 1 << v;
+  return czt_is_blk(v) ? v : 0;
+}
+
+static int dispatch_rows(cudaStream_t st, const CztLaunch& p, int len) {
+  if (czt_is_blk(len)) {
+    XL_CZT_BLK_DISPATCH(len, czt_blk_rows, st, p)
+  }
+  const int ll = ilog2_ceil(len);
   XL_CZT_DISPATCH(ll, czt_rows_launch, st, p)
-  set_error("czt: unsupported Bluestein length 2^%d", ll);
+  set_error("czt: unsupported Bluestein length %d", len);
   return XL_EUNSUPPORTED;
 }
 
-static int dispatch_cols(cudaStream_t st, const CztLaunch& p, int ll) {
+static int dispatch_cols(cudaStream_t st, const CztLaunch& p, int len) {
+  if (czt_is_blk(len)) {
+    XL_CZT_BLK_DISPATCH(len, czt_blk_cols, st, p)
+  }
+  const int ll = ilog2_ceil(len);
   XL_CZT_DISPATCH(ll, czt_cols_launch, st, p)
-  set_error("czt: unsupported Bluestein length 2^%d", ll);
+  set_error("czt: unsupported Bluestein length %d", len);
   return XL_EUNSUPPORTED;
 }
 
@@ -233,10 +256,10 @@ static int czt_run(void* stream, const XlCztArgs* a, int stage) {
     set_error("xl_czt: mode %d with comps %d -> %d is not supported", a->mode, a->comps_in, a->comps_out);
     return XL_EINVAL;
   }
-  const int llx = a->log2_lx, lly = a->log2_ly;
-  if (llx < 5 || llx > 13 || lly < 5 || lly > 13 || (1 << llx) < a->nx + a->mx ||
-      (1 << lly) < a->ny + a->my) {
-    set_error("xl_czt: Bluestein lengths 2^%d, 2^%d must be in 32..8192 and exceed m + M - 1",
+  const int lx = czt_len(a->log2_lx), ly = czt_len(a->log2_ly);
+  if (lx < a->nx + a->mx || ly < a->ny + a->my ||
+      (a->z_batch && (a->log2_lx > 13 || a->log2_ly > 13))) {
+    set_error("xl_czt: Bluestein lengths (log2 %d, %d, or 512 k) must be in 32..8192 and exceed m + M - 1",
               a->log2_lx, a->log2_ly);
     return XL_EINVAL;
   }
@@ -273,7 +296,7 @@ static int czt_run(void* stream, const XlCztArgs* a, int stage) {
   CztLaunch p;
   p.B = a->batch; p.cin = a->comps_in; p.cout = a->comps_out;
   p.ny = a->ny; p.nx = a->nx; p.my = a->my; p.mx = a->mx; p.mode = a->mode;
-  const int wt = czt_tile_w(lly);
+  const int wt = czt_is_blk(ly) ? 8 : czt_tile_w(ilog2_ceil(ly));
   p.mxp = (a->mx + wt - 1) / wt * wt;
   p.lw = ilog2_ceil(wt);
   p.adjoint = a->adjoint ? 1 : 0;
@@ -298,13 +321,15 @@ static int czt_run(void* stream, const XlCztArgs* a, int stage) {
   p.pre = a->pre;
   p.zb = a->z_batch;
   p.cteb = (const float2*)a->cte_batch;
+  p.nat_x = a->log2_lx <= 13;
+  p.nat_y = a->log2_ly <= 13;
   p.fin = (const float2*)a->f_in;
   p.fout = (const float2*)a->f_out;
   cudaStream_t st = (cudaStream_t)stream;
   if (stage < 0 || stage == 0)
-    if (int rc = dispatch_rows(st, p, llx)) return rc;
+    if (int rc = dispatch_rows(st, p, lx)) return rc;
   if (stage < 0 || stage == 1)
-    if (int rc = dispatch_cols(st, p, lly)) return rc;
+    if (int rc = dispatch_cols(st, p, ly)) return rc;
   return XL_OK;
 }
 

@@ -35,6 +35,7 @@ struct CztLaunch {
   XlProg pre;
   const double* zb;      // per-entry distances (NULL: z for every entry); with them the
   const float2* cteb;    // chirps are packed per entry and cteb[b] replaces cte
+  bool nat_x, nat_y;     // block engine lengths: g_x, g_y in natural order (else in block order)
   const float2* fin;     // transfer function on the input plane (ny x nx), or NULL
   const float2* fout;    // and on the output plane (my x mx), or NULL
 };
@@ -42,6 +43,11 @@ struct CztLaunch {
 // Entry b's chirp vector: the shared one, or its slot in the per-entry packing.
 __device__ __forceinline__ const float2* czt_entry(const float2* v, const CztLaunch& p, int b, int len) {
   return p.zb ? v + (long long)b * len : v;
+}
+
+// Element (row r, column col) of the intermediate, in column tiles of 2^lw.
+__device__ __forceinline__ long long tiled_rt(int r, int col, int rows, int lw) {
+  return ((((long long)(col >> lw)) * rows + r) << lw) + (col & ((1 << lw) - 1));
 }
 
 // Column-tile width of the intermediate, set by the y transform's length 2^logl.
@@ -57,5 +63,11 @@ template <int LOGL>
 int czt_rows_launch(cudaStream_t st, const CztLaunch& p);
 template <int LOGL>
 int czt_cols_launch(cudaStream_t st, const CztLaunch& p);
+
+// The same for the block engine's lengths of 256 R points, R = 4, 6, .. 16
+// (explicitly instantiated in czt_b*.cu).  Its column tiles are 8 wide.
+inline bool czt_is_blk(int len) { return len >= 1024 && len <= 4096 && len % 512 == 0; }
+template <int R> int czt_blk_rows(cudaStream_t st, const CztLaunch& p);
+template <int R> int czt_blk_cols(cudaStream_t st, const CztLaunch& p);
 
 }  // namespace xl

@@ -2,6 +2,9 @@
 // the high-NA objective-lens focus, forward and adjoint; the kernels and their
 // launch code, included by the czt_l*.cu translation units.
 //
+// Lengths of 1024 to 4096 points run in czt_blk.cuh; here are the shorter ones
+// and 8192.
+//
 // The reference (wave_optics.py:333-460) runs Bluestein's algorithm along y
 // and then along x, each as: multiply the input line by a pre-chirp,
 // zero-pad to L = next_pow2(m+M-1), FFT, multiply by the spectrum of the
@@ -54,31 +57,24 @@ template <int LOGL> struct CztCfg {
 // x transform organisation for NC line components: CG component groups of G
 // rows of T threads; CG = NC (every component of a row at once) when the CTA
 // can hold them, else 1.
-template <int LOGL, int NC, bool OG = false> struct CztRowCfg {
+template <int LOGL, int NC> struct CztRowCfg {
   using C = CztCfg<LOGL>;
-  // OG: one component group whatever NC (the components one after the other)
-  static constexpr int CG = (!OG && NC * C::G * C::T <= 1024) ? NC : 1;
+  static constexpr int CG = NC * C::G * C::T <= 1024 ? NC : 1;
   static constexpr int ITER = (NC + CG - 1) / CG;              // transforms per group and row
   static constexpr int LINES = CG * C::G;
   static constexpr int THREADS = LINES * C::T;
   static constexpr int MINB = (768 / THREADS) > 1 ? (768 / THREADS) : 1;
 };
 
-__device__ __forceinline__ long long tiled_rt(int r, int col, int rows, int lw) {
-  return ((((long long)(col >> lw)) * rows + r) << lw) + (col & ((1 << lw) - 1));
-}
-
 // x transform.  NC: components per row (1, or 3 for VCZT and the high-NA
 // focus; a plain transform of 2 components runs as 3 with the third idle).
 // ZU: the input window lies in the first half of the line.  MB: resident
-// CTAs per SM the registers are sized for (0: CztRowCfg's MINB).  FK: the
-// fused program's op kinds fixed at compile time (FixedKinds<...>, for the
-// tables' programs), or FixedKinds<>.
-template <int LOGL, int NC, bool ZU, int MB = 0, class FK = FixedKinds<>, bool OG = false>
-__global__ void __launch_bounds__(CztRowCfg<LOGL, NC, OG>::THREADS, MB ? MB : CztRowCfg<LOGL, NC, OG>::MINB)
+// CTAs per SM the registers are sized for (0: CztRowCfg's MINB).
+template <int LOGL, int NC, bool ZU, int MB = 0>
+__global__ void __launch_bounds__(CztRowCfg<LOGL, NC>::THREADS, MB ? MB : CztRowCfg<LOGL, NC>::MINB)
     czt_rows(const __grid_constant__ CztLaunch p, const __grid_constant__ RowStage st) {
   using C = CztCfg<LOGL>;
-  using F = CztRowCfg<LOGL, NC, OG>;
+  using F = CztRowCfg<LOGL, NC>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = p.nx, ny = p.ny;
   float2* xch = (float2*)smraw;                                    // LINES x XS
@@ -145,8 +141,7 @@ __global__ void __launch_bounds__(CztRowCfg<LOGL, NC, OG>::THREADS, MB ? MB : Cz
         px[q] = PixelCtx{r, n, pix, b};
         pr[q] = StagedParams{stage, &st, g2, nx, n};
       }
-      if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
-      else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
+      if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
 #pragma unroll
       for (int q = 0; q < NPX; ++q) {
         const int r = px[q].row, n = px[q].col;
@@ -168,11 +163,6 @@ __global__ void __launch_bounds__(CztRowCfg<LOGL, NC, OG>::THREADS, MB ? MB : Cz
     };
     {
       int base = tid;
-      // a fixed program with registers for two CTAs per SM (128): eight at a
-      // time first (1932 against 1911 tables/s on the high-NA step)
-      if constexpr (F::THREADS <= 256 && FK::n > 0 && MB == 2) {
-        for (; base + 7 * F::THREADS < lim; base += 8 * F::THREADS) chunk(std::integral_constant<int, 8>{}, base);
-      }
       if constexpr (F::THREADS <= 256) {   // CTAs of 768 threads ran slower with it
         for (; base + 3 * F::THREADS < lim; base += 4 * F::THREADS) chunk(std::integral_constant<int, 4>{}, base);
       }
@@ -325,10 +315,10 @@ __global__ void __launch_bounds__(CztCfg<LOGL>::COL_THREADS, CztCfg<LOGL>::COL_M
 // ---------------------------------------------------------------------------
 // Launch code.
 
-template <int LOGL, int NC, bool ZU, int MB = 0, class FK = FixedKinds<>, bool OG = false>
+template <int LOGL, int NC, bool ZU, int MB = 0>
 static int launch_czt_rows(cudaStream_t s, const CztLaunch& p) {
   using C = CztCfg<LOGL>;
-  using F = CztRowCfg<LOGL, NC, OG>;
+  using F = CztRowCfg<LOGL, NC>;
   const size_t fixed = ((size_t)(F::LINES * C::XS + NC * C::G * p.nx) * 8 + 15) / 16 * 16;
   // kernel variant: 0 cap the stage so that two CTAs fit per SM where the
   // registers allow two (the one-component transforms; three components keep
@@ -336,22 +326,13 @@ static int launch_czt_rows(cudaStream_t s, const CztLaunch& p) {
   // that fits one CTA per SM; 2 stage nothing (all planes read from global
   // memory, as many CTAs as the registers allow); 3 as 0 with the registers
   // sized for two CTAs per SM instead of three (MB = 2: no spills).
-  // Measured on the Ez-only high-NA step (32 x 2048^2): 1354 (0), 1138 (1),
-  // 1348 (2) tables/s.
-  // 4 (three components, 4096 points): one component group transforming
-  // the components one after the other, two CTAs per SM as in 3.
-  int var = kernel_variant(XL_PASS_CZT_ROWS, LOGL);
-  if (var == 4 && NC == 1) var = 3;   // a single component is one group already
-  if constexpr (NC == 3 && LOGL == 12 && !OG) {
-    if (var == 4) return launch_czt_rows<LOGL, NC, ZU, 2, FK, true>(s, p);
-  }
+  const int var = kernel_variant(XL_PASS_CZT_ROWS, LOGL);
   constexpr int MB2 = 512 / F::THREADS;   // two CTAs of 256 threads
   if constexpr (NC == 1 && MB == 0 && MB2 >= 1 && MB2 < F::MINB) {
-    if (var == 3) return launch_czt_rows<LOGL, NC, ZU, MB2, FK>(s, p);
+    if (var == 3) return launch_czt_rows<LOGL, NC, ZU, MB2>(s, p);
   }
   const size_t one_cta = (size_t)226 * 1024, two_cta = (size_t)(227 * 1024) / 2 - 1024;
-  const size_t cap = (var == 0 || var == 3 || var == 4) ? ((NC == 1 || OG) ? two_cta : one_cta)
-                     : var == 1 ? one_cta : 0;
+  const size_t cap = (var == 0 || var == 3) ? (NC == 1 ? two_cta : one_cta) : var == 1 ? one_cta : 0;
   RowStage st;
   plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, C::G, fixed, st, cap);
   const size_t sm = fixed + (size_t)C::G * st.row_bytes + 16;
@@ -360,10 +341,10 @@ static int launch_czt_rows(cudaStream_t s, const CztLaunch& p) {
     return XL_EUNSUPPORTED;
   }
   int per_sm;
-  if (int rc = launch_ready<czt_rows<LOGL, NC, ZU, MB, FK, OG>>(F::THREADS, sm, &per_sm, "czt_rows")) return rc;
+  if (int rc = launch_ready<czt_rows<LOGL, NC, ZU, MB>>(F::THREADS, sm, &per_sm, "czt_rows")) return rc;
   const int total = p.B * ((p.ny + C::G - 1) / C::G);
   const int grid = persistent_grid(per_sm, total);
-  czt_rows<LOGL, NC, ZU, MB, FK, OG><<<grid, F::THREADS, sm, s>>>(p, st);
+  czt_rows<LOGL, NC, ZU, MB><<<grid, F::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("czt_rows");
   return XL_OK;
 }
@@ -371,24 +352,7 @@ static int launch_czt_rows(cudaStream_t s, const CztLaunch& p) {
 template <int LOGL>
 int czt_rows_launch(cudaStream_t s, const CztLaunch& p) {
   const bool zu = p.ioff_x >= 0 && p.ioff_x + p.nx <= (1 << LOGL) / 2;
-  // the tables' forward programs get a kernel with their op kinds fixed: the
-  // high-NA table's LCD, sSLM and lens Ez row (4096-point lines), the 4f
-  // table's thin lens (2048-point lines) and second phase SLM (1024-point)
-  if constexpr (LOGL == 12) {
-    using HighNaEz = FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ>;
-    if (p.cout == 1 && zu && HighNaEz::matches(p.pre)) return launch_czt_rows<LOGL, 1, true, 0, HighNaEz>(s, p);
-  }
-  if constexpr (LOGL == 11) {
-    using LensOnly = FixedKinds<XL_OP_SEPMASK>;
-    if (p.cout == 1 && zu && LensOnly::matches(p.pre)) return launch_czt_rows<LOGL, 1, true, 0, LensOnly>(s, p);
-  }
-  if constexpr (LOGL == 10) {
-    using SlmOnly = FixedKinds<XL_OP_PHASE>;
-    if (p.cout == 1 && zu && SlmOnly::matches(p.pre)) return launch_czt_rows<LOGL, 1, true, 0, SlmOnly>(s, p);
-  }
   if (p.cout == 1) return zu ? launch_czt_rows<LOGL, 1, true>(s, p) : launch_czt_rows<LOGL, 1, false>(s, p);
-  // (a fixed LCD-sSLM-lens program in the three-component kernel ran slower:
-  // 1.96 against 1.90 ms per 8 x 2048^2 high-NA focuses)
   return zu ? launch_czt_rows<LOGL, 3, true>(s, p) : launch_czt_rows<LOGL, 3, false>(s, p);
 }
 

@@ -69,6 +69,7 @@ struct RowStage {
   int row_bytes;               // sum of the streams' row bytes
   RowStream s[XL_ROW_STREAMS];
   int fld[3];                  // stage offset of input component c, -1: read from global memory
+  int aux;                     // stage offset of a caller's plane of complex values, -1: global memory
   int prm[XL_MAX_OPS][4];      // stage offset of parameter plane i of op k, -1: global memory
   // planes the prologue reads from global memory (not staged, or the lens
   // coefficient planes); the chirp-z x transform prefetches them into L2 one
@@ -119,7 +120,8 @@ __device__ __forceinline__ void prefetch_rows(const RowStage& st, int b, int r0,
 // CTA's shared memory, barrier included; a smaller cap leaves room for more
 // CTAs per SM, the planes that do not fit are read from global memory).
 static inline void plan_row_stage(int cin, const float2* const* in, long long ibs, int nx, const XlProg& prog,
-                                  int G, size_t fixed_smem, RowStage& st, size_t cap = 226 * 1024) {
+                                  int G, size_t fixed_smem, RowStage& st, size_t cap = 226 * 1024,
+                                  const float2* aux = nullptr) {
   st.n = 0;
   st.row_bytes = 0;
   for (int c = 0; c < 3; ++c) st.fld[c] = -1;
@@ -156,6 +158,8 @@ static inline void plan_row_stage(int cin, const float2* const* in, long long ib
     st.fld[c] = add(in[c], ibs * 8, nx * 8);
     if (st.fld[c] < 0) prefetch(in[c], ibs * 8, nx * 8);
   }
+  st.aux = add(aux, 0, nx * 8);
+  if (st.aux < 0) prefetch(aux, 0, nx * 8);
   for (int k = 0; k < prog.nops; ++k) {
     const XlOp& op = prog.ops[k];
     for (int i = 0; i < 4; ++i)

@@ -808,15 +808,43 @@ def _per_entry(z):
     return isinstance(z, (list, tuple, np.ndarray)) and np.ndim(z) >= 1
 
 
-def bluestein_plan(m, f1, f2, Dm, M):
+def czt_length(m, M):
+    """The length the chirp-z kernels run an m-point line onto M outputs at:
+    the shortest of 1024, 1536, .. 4096 that holds the m + M points (the result
+    does not depend on it), or the reference's power of two outside that range."""
+    Lk = bluestein_length(m, M)
+    return Lk if Lk < 1024 or Lk > 4096 else max(1024, -(-(m + M) // 512) * 512)
+
+
+def _is_block_length(L):
+    return 1024 <= L <= 4096 and L % 512 == 0
+
+
+def _length_code(L, per_entry=False):
+    """A Bluestein length as XlCztArgs takes it: itself for the lengths whose
+    spectrum is passed in block order, else log2."""
+    L = int(L)
+    return L if _is_block_length(L) and not per_entry else L.bit_length() - 1
+
+
+def _block_order(L):
+    """Natural index of each entry of a spectrum in block order (xlgb.h): entry
+    m 16 R + 16 k1 + k2 is k1 + R (k2 + 16 m), L = 256 R."""
+    R = L // 256
+    m, k1, k2 = np.arange(16)[:, None, None], np.arange(R)[None, :, None], np.arange(16)[None, None, :]
+    return (k1 + R * (k2 + 16 * m)).reshape(-1)
+
+
+def bluestein_plan(m, f1, f2, Dm, M, length=None):
     """Chirp data of wave_optics.py:385-460 for an m-point input and M outputs, float64.
+    ``length``: the transform length (the reference's if None).
 
     Returns (L, pre, g, post): L the transform length; pre[n] = A^-n
     h[m-1+n]; g = fft(1/h[:m+M], L) in natural order;
     post[l] = h[m-1+l] exp(-i 2 pi l_f (1/2 - m/2) / Dm) / L, where
     h[q] = W^((q-m+1)^2/2) with the complex power's principal branch.
     """
-    Lk = bluestein_length(m, M)
+    Lk = length or bluestein_length(m, M)
     D1 = f1 + (M * Dm + f2 - f1) / (2 * M)
     D2 = f2 + (M * Dm + f2 - f1) / (2 * M)
     mp = m + M - 1
@@ -834,9 +862,11 @@ def bluestein_plan(m, f1, f2, Dm, M):
 _chirp_cache: "collections.OrderedDict" = collections.OrderedDict()
 
 
-def device_chirps(m, f1, f2, Dm, M, adjoint=False):
-    """Chirp vectors on the device; the adjoint set is (conj(post) L, conj(g), conj(pre) / L)."""
-    key = (int(m), float(f1), float(f2), float(Dm), int(M), bool(adjoint), torch.cuda.current_device())
+def device_chirps(m, f1, f2, Dm, M, adjoint=False, length=None):
+    """Chirp vectors on the device; the adjoint set is (conj(post) L, conj(g), conj(pre) / L).
+    With a ``length`` (czt_length's) the spectrum g comes in the order the
+    kernels of that length read it."""
+    key = (int(m), float(f1), float(f2), float(Dm), int(M), bool(adjoint), length, torch.cuda.current_device())
     with _LOCK:
         v = _chirp_cache.get(key)
         if v is not None:
@@ -844,9 +874,11 @@ def device_chirps(m, f1, f2, Dm, M, adjoint=False):
             for t in v[1:]:
                 keep_for_capture(t)
             return v
-    L, pre, g, post = bluestein_plan(m, f1, f2, Dm, M)
+    L, pre, g, post = bluestein_plan(m, f1, f2, Dm, M, length)
     if adjoint:
         pre, g, post = np.conj(post) * L, np.conj(g), np.conj(pre) / L
+    if length and _is_block_length(L):
+        g = g[_block_order(L)]
     dev = device()
     v = (L,) + tuple(torch.as_tensor(a, device=dev).to(torch.complex64) for a in (pre, g, post))
     with _LOCK:
@@ -969,8 +1001,10 @@ class CztCall:
             Lx, Ly, prex, gx, postx, prey, gy, posty, cteb = entry_chirps(zb, wavelength, x, y, xout, yout, adjoint)
             cte, zz = 0.0, 0.0
         else:
-            Lx, prex, gx, postx = device_chirps(nx, xout[0] + Dm / 2, xout[-1] + Dm / 2, Dm, mx, adjoint)
-            Ly, prey, gy, posty = device_chirps(ny, yout[0] + Dm / 2, yout[-1] + Dm / 2, Dm, my, adjoint)
+            Lx, prex, gx, postx = device_chirps(nx, xout[0] + Dm / 2, xout[-1] + Dm / 2, Dm, mx, adjoint,
+                                                  czt_length(nx, mx))
+            Ly, prey, gy, posty = device_chirps(ny, yout[0] + Dm / 2, yout[-1] + Dm / 2, Dm, my, adjoint,
+                                                  czt_length(ny, my))
         if adjoint:   # the call reads the forward's output plane and writes its input plane
             x, y, xout, yout = xout, yout, x, y
             ny, nx, my, mx = my, mx, ny, nx
@@ -982,7 +1016,7 @@ class CztCall:
         a.batch, a.comps_in, a.comps_out, a.mode = B, cin, cout, cmode
         a.ny, a.nx, a.my, a.mx = ny, nx, my, mx
         a.adjoint = 1 if adjoint else 0
-        a.log2_lx, a.log2_ly = int(Lx).bit_length() - 1, int(Ly).bit_length() - 1
+        a.log2_lx, a.log2_ly = _length_code(Lx, zb is not None), _length_code(Ly, zb is not None)
         for i, c in enumerate(comps):
             a.inp[i] = c.data_ptr()
         for i, o in enumerate(outs):
@@ -1031,15 +1065,15 @@ def czt_plain(comps, mx, my, Dm, fy1, fy2, fx1, fx2, cte=1.0):
     lead = comps[0].shape[:-2]
     planes, B, ibs = batch_planes(comps, ny, nx)
     dev = planes[0].device
-    Lx, prex, gx, postx = device_chirps(nx, float(fx1), float(fx2), float(Dm), int(mx))
-    Ly, prey, gy, posty = device_chirps(ny, float(fy1), float(fy2), float(Dm), int(my))
+    Lx, prex, gx, postx = device_chirps(nx, float(fx1), float(fx2), float(Dm), int(mx), length=czt_length(nx, int(mx)))
+    Ly, prey, gy, posty = device_chirps(ny, float(fy1), float(fy2), float(Dm), int(my), length=czt_length(ny, int(my)))
     C = len(planes)
     work = torch.empty(L.xl_czt_work_bytes(B, C, ny, mx) // 8, dtype=torch.complex64, device=dev)
     outs = [torch.empty(tuple(lead) + (my, mx), dtype=torch.complex64, device=dev) for _ in range(C)]
     a = _lib.XlCztArgs()
     a.batch, a.comps_in, a.comps_out, a.mode = B, C, C, _lib.XL_CZT_PLAIN
     a.ny, a.nx, a.my, a.mx = ny, nx, int(my), int(mx)
-    a.log2_lx, a.log2_ly = int(Lx).bit_length() - 1, int(Ly).bit_length() - 1
+    a.log2_lx, a.log2_ly = _length_code(Lx), _length_code(Ly)
     for i, c in enumerate(planes):
         a.inp[i] = c.data_ptr()
     for i, o in enumerate(outs):
