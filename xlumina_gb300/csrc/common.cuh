@@ -223,15 +223,15 @@ struct GlobalParams {
 };
 
 // The LCD retarder (delta = 0) from cos, sin of eta/2 and of theta:
-// a = ch - i sh (c^2 - s^2), b = c = -i sh 2 s c, d = ch + i sh (c^2 - s^2).
+// J = ch - i sh M with M = [[c2, s2], [s2, -c2]], c2 = cos 2 theta, s2 = sin 2
+// theta, so J e = ch e - i sh (M e): sixteen multiply-adds.
 __device__ __forceinline__ void lcd_apply_trig(float ch, float sh, float ct, float st, float2 (&e)[3]) {
   const float c2 = ct * ct - st * st, s2 = 2.f * st * ct;
-  const float2 a = make_float2(ch, -sh * c2);
-  const float2 b = make_float2(0.f, -sh * s2);
-  const float2 d = make_float2(ch, sh * c2);
   const float2 x = e[0], y = e[1];
-  e[0] = cadd(cmul(a, x), cmul(b, y));
-  e[1] = cadd(cmul(b, x), cmul(d, y));
+  const float2 w0 = make_float2(c2 * x.x + s2 * y.x, c2 * x.y + s2 * y.y);
+  const float2 w1 = make_float2(s2 * x.x - c2 * y.x, s2 * x.y - c2 * y.y);
+  e[0] = make_float2(ch * x.x + sh * w0.y, ch * x.y - sh * w0.x);
+  e[1] = make_float2(ch * y.x + sh * w1.y, ch * y.y - sh * w1.x);
 }
 
 // Op k of a program applied to one pixel's (Ex, Ey, Ez) (scalar fields use
@@ -408,23 +408,26 @@ __device__ __forceinline__ void apply_prog(const XlProg& prog, float2 (&e)[3], c
 // dL/dp = Re(sum_c g_c conj(dy_c/dp)).
 __device__ __forceinline__ float re_gconj(float2 g, float2 d) { return g.x * d.x + g.y * d.y; }
 
+// Re(g conj(i x)): the gradient along a phase of x.
+__device__ __forceinline__ float re_gconj_i(float2 g, float2 x) { return g.y * x.x - g.x * x.y; }
+
 // Backward of lcd_apply_trig: parameter gradients into pg[0] (eta), pg[1]
-// (theta); g becomes J^H g (J symmetric: conj(J) g).
+// (theta); g becomes J^H g = ch g + i sh M g.  With P = Re<g, e>,
+// B_kl = Re(g_k conj(i e_l)), D = B_00 - B_11 and S = B_01 + B_10,
+// dL/deta = -(sh P + ch (c2 D + s2 S)) / 2 and dL/dtheta = -2 sh (c2 S - s2 D).
 __device__ __forceinline__ void lcd_bwd_trig(float ch, float sh, float ct, float st, const float2 (&e)[3],
                                              float2 (&g)[3], float (&pg)[4]) {
   const float c2 = ct * ct - st * st, s2 = 2.f * st * ct;
-  const float2 a = make_float2(ch, -sh * c2), bb = make_float2(0.f, -sh * s2), d = make_float2(ch, sh * c2);
-  // derivatives of the matrix entries
-  const float2 a_e = make_float2(-0.5f * sh, -0.5f * ch * c2), b_e = make_float2(0.f, -0.5f * ch * s2);
-  const float2 d_e = make_float2(-0.5f * sh, 0.5f * ch * c2);
-  const float2 a_t = make_float2(0.f, 2.f * sh * s2), b_t = make_float2(0.f, -2.f * sh * c2);
-  const float2 d_t = make_float2(0.f, -2.f * sh * s2);
-  const float2 x = e[0], y = e[1];
-  pg[0] += re_gconj(g[0], cadd(cmul(a_e, x), cmul(b_e, y))) + re_gconj(g[1], cadd(cmul(b_e, x), cmul(d_e, y)));
-  pg[1] += re_gconj(g[0], cadd(cmul(a_t, x), cmul(b_t, y))) + re_gconj(g[1], cadd(cmul(b_t, x), cmul(d_t, y)));
   const float2 g0 = g[0], g1 = g[1];
-  g[0] = cadd(cmul(cconj(a), g0), cmul(cconj(bb), g1));
-  g[1] = cadd(cmul(cconj(bb), g0), cmul(cconj(d), g1));
+  const float P = re_gconj(g0, e[0]) + re_gconj(g1, e[1]);
+  const float D = re_gconj_i(g0, e[0]) - re_gconj_i(g1, e[1]);
+  const float S = re_gconj_i(g0, e[1]) + re_gconj_i(g1, e[0]);
+  pg[0] -= 0.5f * (sh * P + ch * (c2 * D + s2 * S));
+  pg[1] -= 2.f * sh * (c2 * S - s2 * D);
+  const float2 v0 = make_float2(c2 * g0.x + s2 * g1.x, c2 * g0.y + s2 * g1.y);
+  const float2 v1 = make_float2(s2 * g0.x - c2 * g1.x, s2 * g0.y - c2 * g1.y);
+  g[0] = make_float2(ch * g0.x - sh * v0.y, ch * g0.y + sh * v0.x);
+  g[1] = make_float2(ch * g1.x - sh * v1.y, ch * g1.y + sh * v1.x);
 }
 
 // The sines and cosines an op's forward and backward need, so that a caller
@@ -433,31 +436,36 @@ __device__ __forceinline__ void lcd_bwd_trig(float ch, float sh, float ct, float
 // of theta; LP (c0, s0) of alpha.  Scalar parameters take the host's values.
 // The kind is passed apart from the op so that a kernel specialised for a
 // fixed program folds the switches below (the generic callers pass op.kind).
-__device__ __forceinline__ float4 op_trig(int kind, const XlOp& op, const PixelCtx& px) {
+// param(i) reads the op's parameter i.
+template <class P>
+__device__ __forceinline__ float4 op_trig_p(int kind, const XlOp& op, const P& param) {
   float4 t = make_float4(1.f, 0.f, 1.f, 0.f);   // (c0, s0, c1, s1)
   switch (kind) {
     case XL_OP_PHASE:
-      phase_sincos(op_param(op, 0, px), &t.y, &t.x);
+      phase_sincos(param(0), &t.y, &t.x);
       break;
     case XL_OP_SSLM:
     case XL_OP_SSLM_AMP:
-      phase_sincos(op_param(op, 0, px), &t.y, &t.x);
-      phase_sincos(op_param(op, 1, px), &t.w, &t.z);
+      phase_sincos(param(0), &t.y, &t.x);
+      phase_sincos(param(1), &t.w, &t.z);
       break;
     case XL_OP_LCD:
-      if (op.pmask & 1) phase_sincos(0.5f * op_param(op, 0, px), &t.y, &t.x);
+      if (op.pmask & 1) phase_sincos(0.5f * param(0), &t.y, &t.x);
       else { t.x = op.dval[0]; t.y = op.dval[1]; }
-      if (op.pmask & 2) phase_sincos(op_param(op, 1, px), &t.w, &t.z);
+      if (op.pmask & 2) phase_sincos(param(1), &t.w, &t.z);
       else { t.z = op.dval[2]; t.w = op.dval[3]; }
       break;
     case XL_OP_LP:
-      if (op.pmask & 1) phase_sincos(op_param(op, 0, px), &t.y, &t.x);
+      if (op.pmask & 1) phase_sincos(param(0), &t.y, &t.x);
       else { t.x = op.sval[2]; t.y = op.sval[3]; }
       break;
     default:
       break;
   }
   return t;
+}
+__device__ __forceinline__ float4 op_trig(int kind, const XlOp& op, const PixelCtx& px) {
+  return op_trig_p(kind, op, [&](int i) { return op_param(op, i, px); });
 }
 __device__ __forceinline__ float4 op_trig(const XlOp& op, const PixelCtx& px) { return op_trig(op.kind, op, px); }
 
@@ -500,27 +508,24 @@ __device__ __forceinline__ void apply_op_bwd_t(int kind, const XlOp& op, const f
                                                float2 (&g)[3], const PixelCtx& px, float (&pg)[4]) {
   switch (kind) {
     case XL_OP_PHASE: {
-      const float2 ph = make_float2(t.x, t.y);
-      const float2 y = cmul(e[0], ph);
-      pg[0] += re_gconj(g[0], make_float2(-y.y, y.x));   // dy/dphi = i y
-      g[0] = cmulc(g[0], ph);
+      // dy/dphi = i y; g and y turned back by the phase give the same product
+      g[0] = cmulc(g[0], make_float2(t.x, t.y));
+      pg[0] += re_gconj_i(g[0], e[0]);
       break;
     }
     case XL_OP_SSLM:
     case XL_OP_SSLM_AMP: {
       const bool amp = kind == XL_OP_SSLM_AMP;
-      const float2 p0 = make_float2(t.x, t.y);
-      const float2 p1 = make_float2(t.z, t.w);
+      const float2 b0 = cmulc(g[0], make_float2(t.x, t.y)), b1 = cmulc(g[1], make_float2(t.z, t.w));
       const float a1 = amp ? op_param(op, 2, px) : 1.f, a2 = amp ? op_param(op, 3, px) : 1.f;
-      const float2 u0 = cmul(e[0], p0), u1 = cmul(e[1], p1);   // before the amplitudes
-      pg[0] += a1 * re_gconj(g[0], make_float2(-u0.y, u0.x));
-      pg[1] += a2 * re_gconj(g[1], make_float2(-u1.y, u1.x));
+      pg[0] += a1 * re_gconj_i(b0, e[0]);
+      pg[1] += a2 * re_gconj_i(b1, e[1]);
       if (amp) {
-        pg[2] += re_gconj(g[0], u0);
-        pg[3] += re_gconj(g[1], u1);
+        pg[2] += re_gconj(b0, e[0]);
+        pg[3] += re_gconj(b1, e[1]);
       }
-      g[0] = cscale(cmulc(g[0], p0), a1);
-      g[1] = cscale(cmulc(g[1], p1), a2);
+      g[0] = cscale(b0, a1);
+      g[1] = cscale(b1, a2);
       break;
     }
     case XL_OP_LCD:

@@ -1,6 +1,7 @@
 // Stand-alone per-pixel kernels: a Jones program applied outside a
 // propagator (masks whose result the caller reads directly).
 #include <initializer_list>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -60,7 +61,9 @@ struct OpsBwdLaunch {
 // programs the tables run), so that the per-op switches fold and the trig
 // stays in registers; FixedKinds<> reads them from the program.
 
-template <int KMAX, class FK = FixedKinds<>>
+// IN: the input's gradient is wanted (otherwise the first op's part of it is not
+// formed).
+template <int KMAX, bool IN, class FK = FixedKinds<>>
 __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p, int scalar_acc, int plane_acc) {
   constexpr int NS = XL_MAX_OPS * 4;
   constexpr int NT = 128;
@@ -107,6 +110,29 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
       e[0] = p.in[0][off];
       if (p.C > 1 && p.in[1]) e[1] = p.in[1][off];
       if (p.C > 2 && p.in[2]) e[2] = p.in[2][off];
+      float2 g[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      const long long go = (long long)b * p.gbs + i;
+      float pv[KMAX][2];
+      if constexpr (FIXED) {
+        // every load of the pixel before the first sine: their slow paths are
+        // branches, past which no load is moved up, and each op's loads were
+        // waited for by themselves (8 x 2048^2 LCD, sSLM, lens Ez row: 589 us,
+        // now 485; LCD and polarizer 448 and 352)
+        g[0] = p.gout[0][go];
+        if (p.C > 1 && p.gout[1]) g[1] = p.gout[1][go];
+        if (p.C > 2 && p.gout[2]) g[2] = p.gout[2][go];
+#pragma unroll
+        for (int k = 0; k < KMAX; ++k)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (kind(k) == XL_OP_LCD || kind(k) == XL_OP_SSLM || (q == 0 && (kind(k) == XL_OP_PHASE || kind(k) == XL_OP_LP)))
+              pv[k][q] = op_param(p.prog.ops[k], q, px);
+      }
+      auto trig_of = [&](int k) {
+        const XlOp& op = p.prog.ops[k];
+        if constexpr (FIXED) return op_trig_p(kind(k), op, [&](int q) { return pv[k][q]; });
+        else return op_trig(kind(k), op, px);
+      };
       // forward recompute: the input of every op (the last op's output is not needed)
 #pragma unroll
       for (int k = 0; k < KMAX; ++k) {
@@ -117,7 +143,7 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
               if (kind(k) == XL_OP_HIGHNA) apply_highna(kc, e);
               else apply_highna_ez(kc, e);
             } else if (k < KMAX - 1) {
-              const float4 t = op_trig(kind(k), p.prog.ops[k], px);
+              const float4 t = trig_of(k);
               if constexpr (FIXED) trig_r[k] = t;
               else trig_s[FIXED ? 0 : k][tid] = t;
               apply_op_t(kind(k), p.prog.ops[k], t, e, px);
@@ -125,11 +151,11 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
           }
         }
       }
-      float2 g[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      const long long go = (long long)b * p.gbs + i;
-      g[0] = p.gout[0][go];
-      if (p.C > 1 && p.gout[1]) g[1] = p.gout[1][go];
-      if (p.C > 2 && p.gout[2]) g[2] = p.gout[2][go];
+      if constexpr (!FIXED) {
+        g[0] = p.gout[0][go];
+        if (p.C > 1 && p.gout[1]) g[1] = p.gout[1][go];
+        if (p.C > 2 && p.gout[2]) g[2] = p.gout[2][go];
+      }
 #pragma unroll
       for (int k = KMAX - 1; k >= 0; --k) {
         if (k < K) {
@@ -142,7 +168,7 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
           }
           else if (k + 1 < K && k < KMAX - 1)
             apply_op_bwd_t(kind(k), op, FIXED ? trig_r[k] : trig_s[FIXED ? 0 : k][tid], ek, g, px, pg);
-          else apply_op_bwd(kind(k), op, ek, g, px, pg);
+          else apply_op_bwd_t(kind(k), op, trig_of(k), ek, g, px, pg);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             void* dst = p.pgrad[k * 4 + q];
@@ -156,10 +182,12 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
           }
         }
       }
-      const long long gi = (long long)b * p.ginbs + i;
-      if (p.gin[0]) p.gin[0][gi] = g[0];
-      if (p.C > 1 && p.gin[1]) p.gin[1][gi] = g[1];
-      if (p.C > 2 && p.gin[2]) p.gin[2][gi] = g[2];
+      if constexpr (IN) {
+        const long long gi = (long long)b * p.ginbs + i;
+        if (p.gin[0]) p.gin[0][gi] = g[0];
+        if (p.C > 1 && p.gin[1]) p.gin[1][gi] = g[1];
+        if (p.C > 2 && p.gin[2]) p.gin[2][gi] = g[2];
+      }
     }
     if (plane_acc)
       for (int k = 0; k < K; ++k)
@@ -188,6 +216,93 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
       }
       __syncthreads();
     }
+}
+
+// Scalar programs of one op, two pixels a thread in 16-byte accesses: a phase
+// SLM with its gradient in a plane per batch entry, and a separable mask (no
+// parameter gradient; the forward's input is not read).  The kernel above, one
+// pixel a thread, does not keep enough bytes in flight: 16 x 1024^2, phase 107
+// us, mask 95; these take 64 and 48 (24 bytes a pixel and 16 at the copy rate: 59
+// and 40).
+template <bool IN>
+__global__ void __launch_bounds__(256) phase_backward_kernel(const OpsBwdLaunch p) {
+  const long long n2 = (long long)p.ny * p.nx / 2;
+  const int b = blockIdx.y;
+  const XlOp& op = p.prog.ops[0];
+  const float4* e2 = (const float4*)(p.in[0] + (long long)b * p.ibs);
+  const float4* g2 = (const float4*)(p.gout[0] + (long long)b * p.gbs);
+  const float2* f2 = (const float2*)((const float*)op.ptr[0] + (long long)b * op.pbstride);
+  float2* d2 = (float2*)((float*)p.pgrad[0] + (long long)b * op.pbstride);
+  float4* o2 = (float4*)(p.gin[0] + (long long)b * p.ginbs);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += (long long)gridDim.x * blockDim.x) {
+    const float4 e = e2[i], g = g2[i];
+    const float2 f = f2[i];
+    float2 s, c;
+    phase_sincos(f.x, &s.x, &c.x);
+    phase_sincos(f.y, &s.y, &c.y);
+    const float2 a = cmulc(make_float2(g.x, g.y), make_float2(c.x, s.x));
+    const float2 h = cmulc(make_float2(g.z, g.w), make_float2(c.y, s.y));
+    d2[i] = make_float2(re_gconj_i(a, make_float2(e.x, e.y)), re_gconj_i(h, make_float2(e.z, e.w)));
+    if constexpr (IN) o2[i] = make_float4(a.x, a.y, h.x, h.y);
+  }
+}
+
+// tc + tr < 1 as float64 arithmetic gives it.  GB300's FP64 pipe takes 16 cycles
+// a warp and operation (it was 79 % busy with two a pixel), so the sum is
+// formed in float from the operands' bits (truncated, within 1e-6) and float64
+// is used only where that is within 1e-4 of 1, or an operand is negative, not
+// finite or huge.
+__device__ __forceinline__ bool pupil_inside(double tc, double tr) {
+  auto bits = [](double v) -> float {   // 0 below 2^-126
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    return hi < (897 << 20) ? 0.f : __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)lo >> 29));
+  };
+  constexpr unsigned BIG = 1150u << 20;   // the high word of 2^127; above it negative values, infinities, NaNs
+  if ((unsigned)__double2hiint(tc) < BIG && (unsigned)__double2hiint(tr) < BIG) {
+    const float s = bits(tc) + bits(tr);
+    if (s < 0.9999f) return true;
+    if (s > 1.0001f) return false;
+  }
+  return tc + tr < 1.0;
+}
+
+__global__ void __launch_bounds__(256) sepmask_backward_kernel(const OpsBwdLaunch p) {
+  const unsigned n2 = (unsigned)((long long)p.ny * p.nx / 2), half = (unsigned)p.nx / 2;
+  const int b = blockIdx.y;
+  const XlOp& op = p.prog.ops[0];
+  const float4* g2 = (const float4*)(p.gout[0] + (long long)b * p.gbs);
+  float4* o2 = (float4*)(p.gin[0] + (long long)b * p.ginbs);
+  const float2* fc = (const float2*)op.ptr[0];
+  const float2* fr = (const float2*)op.ptr[1];
+  const double* tc = (const double*)op.ptr[2];
+  const double* tr = (const double*)op.ptr[3];
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += gridDim.x * blockDim.x) {
+    const unsigned row = i / half, col = 2 * (i - row * half);
+    const float4 g = g2[i];
+    float2 m0 = cmul(fc[col], fr[row]), m1 = cmul(fc[col + 1], fr[row]);
+    if (tc) {
+      const double t = tr[row];
+      if (!pupil_inside(tc[col], t)) m0 = make_float2(0.f, 0.f);
+      if (!pupil_inside(tc[col + 1], t)) m1 = make_float2(0.f, 0.f);
+    }
+    const float2 a = cmulc(make_float2(g.x, g.y), m0), h = cmulc(make_float2(g.z, g.w), m1);
+    o2[i] = make_float4(a.x, a.y, h.x, h.y);
+  }
+}
+
+// Whether one of the two kernels above takes a launch: scalar, one op of its
+// kind, planes and strides that keep every pair 16-byte (parameters: 8-byte)
+// aligned, a phase plane per entry (its gradient needs no sum over the batch).
+static bool pairs_ok(const OpsBwdLaunch& p) {
+  if (p.C != 1 || p.prog.nops != 1 || p.B > 65535) return false;
+  const XlOp& op = p.prog.ops[0];
+  auto al = [](const void* q, int n) { return ((uintptr_t)q % n) == 0; };
+  if (((long long)p.ny * p.nx) % 2 || p.gbs % 2 || !al(p.gout[0], 16)) return false;
+  if (p.gin[0] && (p.ginbs % 2 || !al(p.gin[0], 16))) return false;
+  if (op.kind == XL_OP_PHASE)
+    return (op.pmask & 1) && p.pgrad[0] && (op.pbstride || p.B == 1) && op.pbstride % 2 == 0 && p.ibs % 2 == 0 &&
+           al(p.in[0], 16) && al(op.ptr[0], 8) && al(p.pgrad[0], 8);
+  return op.kind == XL_OP_SEPMASK && p.nx % 2 == 0 && p.gin[0];
 }
 
 __global__ void highna_plane_kernel(int ny, int nx, XlOp op, float* out) {
@@ -491,21 +606,38 @@ extern "C" int xl_ops_backward(void* stream, int batch, int comps, int ny, int n
     return true;
   };
   cudaStream_t s = (cudaStream_t)stream;
+  const bool want_in = p.gin[0] || p.gin[1] || p.gin[2];
+  if (pairs_ok(p)) {
+    // about 16 blocks an SM over the batch, no more than the pairs need
+    long long bx = (npix / 2 + 255) / 256, most = (16LL * sms + batch - 1) / batch;
+    if (bx > most) bx = most;
+    const dim3 grid((unsigned)(bx < 1 ? 1 : bx), batch);
+    if (prog->ops[0].kind == XL_OP_SEPMASK) sepmask_backward_kernel<<<grid, 256, 0, s>>>(p);
+    else if (want_in) phase_backward_kernel<true><<<grid, 256, 0, s>>>(p);
+    else phase_backward_kernel<false><<<grid, 256, 0, s>>>(p);
+    XL_CHECK_LAUNCH("one-op backward");
+    return XL_OK;
+  }
   auto run = [&](auto kernel) { kernel<<<grid_for(kernel), 128, sm, s>>>(p, scalar_acc, plane_acc); };
-  if (is({XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ}))
-    run(ops_backward_kernel<3, FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ>>);
-  else if (is({XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA}))
-    run(ops_backward_kernel<3, FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA>>);
-  else if (is({XL_OP_LCD, XL_OP_LP}))
-    run(ops_backward_kernel<2, FixedKinds<XL_OP_LCD, XL_OP_LP>>);
-  else if (is({XL_OP_PHASE}))
-    run(ops_backward_kernel<1, FixedKinds<XL_OP_PHASE>>);
-  else if (is({XL_OP_SEPMASK}))
-    run(ops_backward_kernel<1, FixedKinds<XL_OP_SEPMASK>>);
-  else if (prog->nops <= 4)
-    run(ops_backward_kernel<4>);
-  else
-    run(ops_backward_kernel<XL_MAX_OPS>);
+  auto pick = [&](auto in) {
+    constexpr bool IN = decltype(in)::value;
+    if (is({XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ}))
+      run(ops_backward_kernel<3, IN, FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ>>);
+    else if (is({XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA}))
+      run(ops_backward_kernel<3, IN, FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA>>);
+    else if (is({XL_OP_LCD, XL_OP_LP}))
+      run(ops_backward_kernel<2, IN, FixedKinds<XL_OP_LCD, XL_OP_LP>>);
+    else if (is({XL_OP_PHASE}))
+      run(ops_backward_kernel<1, IN, FixedKinds<XL_OP_PHASE>>);
+    else if (is({XL_OP_SEPMASK}))
+      run(ops_backward_kernel<1, IN, FixedKinds<XL_OP_SEPMASK>>);
+    else if (prog->nops <= 4)
+      run(ops_backward_kernel<4, IN>);
+    else
+      run(ops_backward_kernel<XL_MAX_OPS, IN>);
+  };
+  if (want_in) pick(std::true_type{});
+  else pick(std::false_type{});
   XL_CHECK_LAUNCH("ops_backward_kernel");
   return XL_OK;
 }
