@@ -227,6 +227,19 @@ static int rs_run(void* stream, const XlRsArgs* a, int stage) {
   // slower (8 x 2048^2 VRS, forward + columns + inverse: 3.5 and 2.8 ms against
   // 2.78; 16 x 1024^2 scalar: 494 and 544 against 470 us)
   p.lw = 3;
+  // Light behind a polarizer at one angle has one transverse degree of freedom:
+  // its Ex and Ey are c and s times one field, and so are their propagations,
+  // so two components are transformed instead of three.
+  p.pol = 0;
+  if (vector && !a->adjoint && a->pre.nops > 0 && a->post.nops == 0 && rs_is_blk(a->ny, a->nx)) {
+    const XlOp& lp = a->pre.ops[a->pre.nops - 1];
+    if (lp.kind == XL_OP_LP && !(lp.pmask & 1)) {
+      p.pol = 1;
+      p.pol_c = lp.sval[2];
+      p.pol_s = lp.sval[3];
+      --p.pre.nops;
+    }
+  }
   cudaStream_t st = (cudaStream_t)stream;
   if (rs_is_blk(a->ny, a->nx)) return blk_propagate(st, p, stage);
   return stockham_propagate(rs_logq(a->ny, a->nx), st, p, stage);

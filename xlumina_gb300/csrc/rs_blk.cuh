@@ -177,39 +177,58 @@ __device__ __forceinline__ long long row_pos(int wq, int lane, int r, int ny, in
   return (((long long)(c >> lw) * ny + r) << lw) + (c & ((1 << lw) - 1));
 }
 
+// Component groups of a forward row CTA: one where a thread runs the program
+// for its own elements, all three for the adjoint.  CTAs per SM the registers
+// are sized for: two of 256 threads where a thread holds a second component
+// (three, 80 registers: 533 us for 8 x 2048^2 fields behind a polarizer, two 467).
+constexpr int rows_fwd_nc(int mode) { return mode == 3 ? 3 : 1; }
+template <int R, int MODE> constexpr int rows_fwd_minb() {
+  return MODE == 1 ? RowB<R, 1>::MINB : (MODE == 3 ? RowB<R, 3>::MINB : 2);
+}
+
 // Bytes of the forward row pass's shared memory before its stage.
 template <int R, int MODE> __host__ __device__ constexpr size_t rows_fwd_fixed(int nx) {
-  using K = RowB<R, MODE == 1 ? 1 : 3>;
-  return ((size_t)(BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE + (MODE == 1 ? 0 : 3 * K::G * nx)) * 8 +
-          (MODE == 2 ? (size_t)nx * 4 : 0) + 15) / 16 * 16;
+  constexpr int NC = rows_fwd_nc(MODE);
+  using K = RowB<R, NC>;
+  constexpr int hold = MODE == 2 ? K::THREADS * BlkFft<R>::IPT * R / 2 : 0;
+  return ((size_t)(BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE + (NC == 1 ? hold : 3 * K::G * nx)) * 8 +
+          (MODE == 2 || MODE == 4 ? (size_t)nx * 4 : 0) + 15) / 16 * 16;
 }
 
 // Forward row pass.  MODE 1: scalar RS (one component); 2: VRS (Ex, Ey in;
-// Ex, Ey, Ez out, Ez derived); 3: VRS adjoint (three gradients in and out).
-// Persistent: CTA c handles row groups c, c + grid, ...  Per row group the
-// prologue runs the fused program over every pixel and writes the components
-// to a shared buffer; the stage is then free, so the bulk copies of the next
-// row group start while the component groups transform this one.  Two CTA
-// barriers a row group: after the prologue, and between the phases A and B.  In
-// a scalar row (MODE 1) the thread that needs an element of phase A runs the
-// program for it itself, so there is no buffer and only the second barrier.
+// Ex, Ey, Ez out, Ez derived); 3: VRS adjoint (three gradients in and out, no
+// program); 4: VRS behind a polarizer at one angle (the program's last op, left
+// out of p.pre): Ex = c u and Ey = s u with u = c Ex' + s Ey', so the row has two
+// components, u and Ez = u (c X + s Y) / r.
+//
+// Persistent: CTA c handles row groups c, c + grid, ...  The thread that needs
+// an element of phase A runs the fused program for it itself, in CTAs of 256
+// threads (several per SM, each at its own point of a row), and transforms its
+// components one after the other; the stage is free after the first phase A and
+// the bulk copies of the next row group start.  (VRS with three component groups
+// in a CTA of 768 threads and the program's results in a shared buffer between:
+// 774 us for 8 x 2048^2 behind an LCD and a polarizer, this form 467 with two
+// components; without a program 694 and WW.)  The adjoint, which has no program,
+// keeps the three groups.
 // FK: the fused program's op kinds fixed at compile time (FixedKinds<...>,
 // for the programs the benchmarks and tables run), or FixedKinds<>.
 template <int R, int MODE, class FK = FixedKinds<>>
-__global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, MODE == 1 ? 1 : 3>::MINB)
+__global__ void __launch_bounds__(RowB<R, rows_fwd_nc(MODE)>::THREADS, rows_fwd_minb<R, MODE>())
     rs_rows_fwd_b(const __grid_constant__ RsLaunch p, const __grid_constant__ RowStage st) {
-  constexpr bool TM = RowB<R, MODE == 1 ? 1 : 3>::TM;
+  constexpr int NC = rows_fwd_nc(MODE);
+  constexpr bool TM = RowB<R, NC>::TM;
   __shared__ unsigned s_tmem;
-  constexpr int NC = MODE == 1 ? 1 : 3;
-  constexpr int CIN = MODE;
+  constexpr int CIN = MODE == 4 ? 2 : MODE;
   using F = BlkFft<R>;
   using K = RowB<R, NC>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = p.nx, ny = p.ny;
   float2* twb = (float2*)smraw;                                      // NTB
   float2* xch = twb + F::NTB;                                        // LINES x LINE
-  float2* post = xch + K::LINES * F::LINE;                           // NC x G x nx (vector modes)
-  float* xf = (float*)(post + (size_t)NC * K::G * nx);               // nx (VRS: x as float32)
+  // the adjoint's rows (3 x G x nx); VRS: Ey of every thread's elements
+  float2* post = xch + K::LINES * F::LINE;
+  constexpr int HOLD = MODE == 2 ? K::THREADS * F::IPT * R / 2 : 0;
+  float* xf = (float*)(post + (NC == 1 ? HOLD : 3 * K::G * nx));     // nx (VRS: x as float32)
   const size_t soff = rows_fwd_fixed<R, MODE>(nx);
   unsigned char* stage = smraw + soff;
   unsigned long long* mbar = (unsigned long long*)(stage + (size_t)K::G * st.row_bytes);
@@ -232,7 +251,7 @@ __global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, M
     fence_mbar_init();
   }
   for (int i = tid; i < F::NTB; i += K::THREADS) twb[i] = blk_tw<R>()[F::NTA + i];
-  if constexpr (MODE == 2)
+  if constexpr (MODE == 2 || MODE == 4)
     for (int i = tid; i < nx; i += K::THREADS) xf[i] = (float)p.x[i];
   __syncthreads();
 
@@ -269,89 +288,60 @@ __global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, M
     const int r = r0 + gi;
     const bool live = r < ny;
     float2 v[16];
-    if constexpr (MODE == 1) {
-      // this thread's elements, four at a time and then the rest; positions
-      // past the row or the field take a valid pixel and are zeroed
+    if constexpr (NC == 1) {
+      // this thread's elements, NP at a time (the program's code is laid out once
+      // for each), through its own slots of the line: no barrier; positions past
+      // the row or the field take a valid pixel and are zeroed
+      constexpr int NP = MODE == 1 ? 4 : 2;
       const int rr = live ? r : ny - 1;
-      auto chunk = [&](auto npx, auto first) {
-        constexpr int NPX = decltype(npx)::value, F0 = decltype(first)::value, H = R / 2;
-        float2 e[NPX][3];
-        PixelCtx px[NPX];
-        StagedParams pr[NPX];
+      constexpr int H = R / 2, N = F::IPT * H;   // 5 to 8 elements
+      float2* own = line + blk_slot(t);
+      auto pos = [&](int f) { return t + f / H * F::T + 256 * (f % H); };
+      auto slot = [&](int f) { return f % H * F::BLK + f / H * (F::T / 16) * 18; };
+#pragma unroll 1
+      for (int f0 = 0; f0 < N; f0 += NP) {
+        float2 e[NP][3];
+        PixelCtx px[NP];
+        StagedParams pr[NP];
 #pragma unroll
-        for (int q = 0; q < NPX; ++q) {
-          const int n = min(t + (F0 + q) / H * F::T + 256 * ((F0 + q) % H), nx - 1);
+        for (int q = 0; q < NP; ++q) {
+          const int n = min(pos(f0 + q), nx - 1);
           const long long pix = (long long)rr * nx + n;
-          const int fo = st.fld[0];
-          e[q][0] = fo >= 0 ? ((const float2*)(stage + fo))[(rr - r0) * nx + n] : p.in[0][(long long)b * p.ibs + pix];
-          e[q][1] = e[q][2] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            e[q][i] = make_float2(0.f, 0.f);
+            if (i < CIN) {
+              const int fo = st.fld[i];
+              e[q][i] = fo >= 0 ? ((const float2*)(stage + fo))[(rr - r0) * nx + n] : p.in[i][(long long)b * p.ibs + pix];
+            }
+          }
           px[q] = PixelCtx{rr, n, pix, b};
           pr[q] = StagedParams{stage, &st, rr - r0, nx, n};
         }
         if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
-        else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
+        else if (p.pre.nops) apply_prog_vec<NP>(p.pre, e, px, pr);
 #pragma unroll
-        for (int q = 0; q < NPX; ++q) {
-          const int f = F0 + q;
-          const bool in = live && t + f / H * F::T + 256 * (f % H) < nx;
-          v[f / H * R + f % H] = in ? e[q][0] : make_float2(0.f, 0.f);
+        for (int q = 0; q < NP; ++q) {
+          if constexpr (MODE == 4) e[q][0] = cadd(cscale(e[q][0], p.pol_c), cscale(e[q][1], p.pol_s));
+          if (N % NP == 0 || f0 + q < N) {
+            own[slot(f0 + q)] = e[q][0];
+            if constexpr (MODE == 2) post[(f0 + q) * K::THREADS + tid] = e[q][1];
+          }
         }
-      };
-      constexpr int N = F::IPT * R / 2;   // 5 to 8
-      chunk(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{});
-      chunk(std::integral_constant<int, N - 4>{}, std::integral_constant<int, 4>{});
+      }
+#pragma unroll
+      for (int f = 0; f < N; ++f)
+        v[f / H * R + f % H] = (live && pos(f) < nx) ? own[slot(f)] : make_float2(0.f, 0.f);
     } else {
       const int lim = min(K::G, ny - r0) * nx;
-      const float zb = MODE == 2 ? (float)p.z[b] : 0.f;
-      // one row per group (2304-point lines and longer): its y and y^2 + z^2
-      // once for the group instead of once per pixel
-      const float Y0 = MODE == 2 && K::G == 1 ? (float)p.y[r0] : 0.f;
-      const float z20 = Y0 * Y0 + zb * zb;
-      auto chunk = [&](auto npx, int base) {
-        constexpr int NPX = decltype(npx)::value;
-        float2 e[NPX][3];
-        PixelCtx px[NPX];
-        StagedParams pr[NPX];
-  #pragma unroll
-        for (int q = 0; q < NPX; ++q) {
-          const int idx = base + q * K::THREADS;
-          const int g2 = K::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, r = r0 + g2;
-          const long long pix = (long long)r * nx + n;
-  #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            e[q][c] = make_float2(0.f, 0.f);
-            if (c < CIN) {
-              const int fo = st.fld[c];
-              e[q][c] = fo >= 0 ? ((const float2*)(stage + fo))[g2 * nx + n] : p.in[c][(long long)b * p.ibs + pix];
-            }
-          }
-          px[q] = PixelCtx{r, n, pix, b};
-          pr[q] = StagedParams{stage, &st, g2, nx, n};
+      for (int idx = tid; idx < lim; idx += K::THREADS) {
+        const int g2 = K::G == 1 ? 0 : idx / nx, n = idx - g2 * nx;
+        const long long pix = (long long)(r0 + g2) * nx + n;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int fo = st.fld[c];
+          post[c * K::G * nx + idx] = fo >= 0 ? ((const float2*)(stage + fo))[idx] : p.in[c][(long long)b * p.ibs + pix];
         }
-        if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
-        else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
-  #pragma unroll
-        for (int q = 0; q < NPX; ++q) {
-          const int r = px[q].row, n = px[q].col;
-          if constexpr (MODE == 2) {  // vectorized_optics.py:258-261, Ez = Ex X/r + Ey Y/r
-            const float Y = K::G == 1 ? Y0 : (float)p.y[r];
-            const float z2 = K::G == 1 ? z20 : Y * Y + zb * zb;
-            const float X = xf[n];
-            const float inv = rsqrtf(X * X + z2);
-            e[q][2] = cadd(cscale(e[q][0], X * inv), cscale(e[q][1], Y * inv));
-          }
-  #pragma unroll
-          for (int c = 0; c < NC; ++c) post[(c * K::G + (r - r0)) * nx + n] = e[q][c];
-        }
-      };
-      {
-        int base = tid;
-        // CTAs of up to 256 threads: four pixels per thread at a time while four
-        // remain, so that their loads and arithmetic overlap and each op of the
-        // program is dispatched once for the four (larger CTAs ran slower so)
-        if constexpr (K::THREADS <= 256)
-          for (; base + 3 * K::THREADS < lim; base += 4 * K::THREADS) chunk(std::integral_constant<int, 4>{}, base);
-        for (; base < lim; base += K::THREADS) chunk(std::integral_constant<int, 1>{}, base);
       }
       // every thread has read the stage and written its pixels; every thread
       // takes the timeout branch or none does
@@ -366,26 +356,70 @@ __global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, M
           v[i * R + n1] = (live && n < nx) ? src[n] : make_float2(0.f, 0.f);
         }
     }
-    blk_a_fwd<R, -1, true>(v, t, line, twa);
-    if constexpr (MODE == 1) {
-      if (__syncthreads_or(!got)) return timed_out();
-      next_stage(grp);
-    } else {
-      __syncthreads();
-    }
-    if (active) {
+    auto finish = [&](int plane) {   // phases B and C of a row, and its store
+      if (!active) return;
       blk_b_fwd<-1>(v, t & 15, blk, twb);
       __syncwarp();
       blk_c_fwd<-1>(v, t & 15, blk);
       if (live) {
-        float2* o = p.work + ((long long)b * NC + cg) * ny * F::P + row_pos(t >> 5, t & 31, r, ny, p.lw);
+        float2* o = p.work + (long long)plane * ny * F::P + row_pos(t >> 5, t & 31, r, ny, p.lw);
         long long step = 32LL * ny;
         asm volatile("" : "+l"(o), "+l"(step));   // one base, not sixteen addresses live across the loop
 #pragma unroll
         for (int q = 0; q < 16; ++q) o[q * step] = v[q];
       }
+    };
+    constexpr bool VRS = MODE == 2 || MODE == 4;
+    float2 uz[VRS ? F::IPT * R / 2 : 1];   // Ez of this thread's elements
+    if constexpr (VRS) {
+      const float zb = (float)p.z[b], Y = (float)p.y[live ? r : ny - 1];
+      const float z2 = Y * Y + zb * zb, sY = p.pol_s * Y;
+#pragma unroll
+      for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+        for (int n1 = 0; n1 < R / 2; ++n1) {   // vectorized_optics.py:258-261, Ez = Ex X/r + Ey Y/r
+          const int f = i * (R / 2) + n1, n = t + i * F::T + 256 * n1;
+          const float X = xf[min(n, nx - 1)], inv = rsqrtf(X * X + z2);
+          if constexpr (MODE == 4) {   // Ex = c u, Ey = s u
+            uz[f] = cscale(v[i * R + n1], (p.pol_c * X + sY) * inv);
+          } else {
+            const float2 ey = live && n < nx ? post[f * K::THREADS + tid] : make_float2(0.f, 0.f);
+            uz[f] = cadd(cscale(v[i * R + n1], X * inv), cscale(ey, Y * inv));
+          }
+        }
     }
-    if constexpr (MODE == 1) __syncthreads();   // the next row's phase A stores to the slots phase C loads here
+    blk_a_fwd<R, -1, true>(v, t, line, twa);
+    if constexpr (NC == 1) {
+      if (__syncthreads_or(!got)) return timed_out();
+      next_stage(grp);
+    } else {
+      __syncthreads();
+    }
+    constexpr int COUT = MODE == 1 ? 1 : (MODE == 4 ? 2 : 3);
+    finish(b * COUT + cg);
+    if constexpr (NC == 1) __syncthreads();   // the next phase A stores to the slots phase C loads here
+    auto another = [&](int c) {   // component c, in v
+      blk_a_fwd<R, -1, true>(v, t, line, twa);
+      __syncthreads();
+      finish(b * COUT + c);
+      __syncthreads();
+    };
+    if constexpr (MODE == 2) {
+#pragma unroll
+      for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+        for (int n1 = 0; n1 < R / 2; ++n1)
+          v[i * R + n1] = live && t + i * F::T + 256 * n1 < nx ? post[(i * (R / 2) + n1) * K::THREADS + tid]
+                                                               : make_float2(0.f, 0.f);
+      another(1);
+    }
+    if constexpr (VRS) {
+#pragma unroll
+      for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+        for (int n1 = 0; n1 < R / 2; ++n1) v[i * R + n1] = uz[i * (R / 2) + n1];
+      another(COUT - 1);
+    }
   }
   if constexpr (TM) tmem_release<K::THREADS, 32>(s_tmem);
 }
@@ -405,7 +439,10 @@ __global__ void __launch_bounds__(RowB<R, MODE == 1 ? 1 : 3>::THREADS, RowB<R, M
 // in Tensor Memory 561; loads that do not allocate in L1 took 628.  Stockham
 // engine: 573.  (16 x 1024^2 scalar, three CTAs an SM: 84 us, 123 on Stockham;
 // with Tensor Memory 95.)
-template <int R, int COUT, bool EPI>
+//
+// POL (one component, no epilogue): the planes u and Ez of VRS behind a
+// polarizer, as entries 2 b and 2 b + 1: Ex = c u, Ey = s u and Ez.
+template <int R, int COUT, bool EPI, bool POL = false>
 __global__ void __launch_bounds__(RowB<R, COUT>::THREADS, RowB<R, COUT>::MINB)
     rs_rows_inv_b(const __grid_constant__ RsLaunch p) {
   constexpr bool TM = RowB<R, COUT>::TM;
@@ -461,7 +498,23 @@ __global__ void __launch_bounds__(RowB<R, COUT>::THREADS, RowB<R, COUT>::MINB)
     else __syncthreads();
     blk_a_inv<R, 1>(v, t, line, twa);
     if constexpr (!EPI) {
-      if (r < ny) {
+      if (POL && r < ny) {
+        const long long row = (long long)(b >> 1) * p.obs + (long long)r * nx;
+        const bool ez = b & 1;
+        float2* o = p.out[ez ? 2 : 0] + row;
+        float2* o1 = p.out[1] + row;
+        const float f = ez ? 1.f : p.pol_c;
+#pragma unroll
+        for (int i = 0; i < F::IPT; ++i)
+#pragma unroll
+          for (int n1 = 0; n1 < R / 2; ++n1) {
+            const int n = t + i * F::T + 256 * n1;
+            if (n < nx) {
+              o[n] = ez ? v[i * R + n1] : cscale(v[i * R + n1], f);
+              if (!ez) o1[n] = cscale(v[i * R + n1], p.pol_s);
+            }
+          }
+      } else if (r < ny) {
         float2* o = p.out[cg] + (long long)b * p.obs + (long long)r * nx;
 #pragma unroll
         for (int i = 0; i < F::IPT; ++i)
@@ -605,10 +658,11 @@ template <int R> static int launch_hhat_cols_b(cudaStream_t st, const float2* in
 
 template <int R, int MODE, class FK = FixedKinds<>>
 static int launch_rows_fwd_b(cudaStream_t s, const RsLaunch& p) {
-  using K = RowB<R, MODE == 1 ? 1 : 3>;
+  using K = RowB<R, rows_fwd_nc(MODE)>;
   const size_t fixed = rows_fwd_fixed<R, MODE>(p.nx);
   RowStage st;
-  plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, K::G, fixed, st);
+  // the stage takes what leaves room for the CTAs the registers allow
+  plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, K::G, fixed, st, (size_t)(227 * 1024) / rows_fwd_minb<R, MODE>() - 1024);
   const size_t sm = fixed + (size_t)K::G * st.row_bytes + 16;
   int per_sm;
   if (int rc = launch_ready<rs_rows_fwd_b<R, MODE, FK>>(K::THREADS, sm, &per_sm, "rs_rows_fwd_b")) return rc;
@@ -619,14 +673,14 @@ static int launch_rows_fwd_b(cudaStream_t s, const RsLaunch& p) {
   return XL_OK;
 }
 
-template <int R, int COUT, bool EPI> static int launch_rows_inv_b(cudaStream_t s, const RsLaunch& p) {
+template <int R, int COUT, bool EPI, bool POL = false> static int launch_rows_inv_b(cudaStream_t s, const RsLaunch& p) {
   using K = RowB<R, COUT>;
   const size_t sm = ((size_t)BlkFft<R>::NTB + K::LINES * BlkFft<R>::LINE) * 8;
   int per_sm;
-  if (int rc = launch_ready<rs_rows_inv_b<R, COUT, EPI>>(K::THREADS, sm, &per_sm, "rs_rows_inv_b")) return rc;
+  if (int rc = launch_ready<rs_rows_inv_b<R, COUT, EPI, POL>>(K::THREADS, sm, &per_sm, "rs_rows_inv_b")) return rc;
   const int total = p.B * ((p.ny + K::G - 1) / K::G);
   const int grid = persistent_grid(per_sm, total);
-  rs_rows_inv_b<R, COUT, EPI><<<grid, K::THREADS, sm, s>>>(p);
+  rs_rows_inv_b<R, COUT, EPI, POL><<<grid, K::THREADS, sm, s>>>(p);
   XL_CHECK_LAUNCH("rs_rows_inv_b");
   return XL_OK;
 }
@@ -634,27 +688,43 @@ template <int R, int COUT, bool EPI> static int launch_rows_inv_b(cudaStream_t s
 template <int R> int rs_blk_rows(cudaStream_t st, const RsLaunch& p, bool inverse) {
   if (!inverse) {
     // the programs of the benchmarks' fields get a kernel with their op kinds
-    // fixed: a phase SLM before scalar RS, an LCD and a polarizer before VRS
+    // fixed: a phase SLM before scalar RS, a double-phase SLM before VRS (the
+    // building block), an LCD before a polarizer and VRS
     using SlmOnly = FixedKinds<XL_OP_PHASE>;
-    using LcdLp = FixedKinds<XL_OP_LCD, XL_OP_LP>;
+    using LcdOnly = FixedKinds<XL_OP_LCD>;
+    if (p.pol) {
+      if constexpr (R >= 8)
+        if (LcdOnly::matches(p.pre)) return launch_rows_fwd_b<R, 4, LcdOnly>(st, p);
+      return launch_rows_fwd_b<R, 4>(st, p);
+    }
     if (p.cout == 1) {
       if constexpr (R >= 8)
         if (SlmOnly::matches(p.pre)) return launch_rows_fwd_b<R, 1, SlmOnly>(st, p);
       return launch_rows_fwd_b<R, 1>(st, p);
     }
+    using SlmsOnly = FixedKinds<XL_OP_SSLM>;
     if (p.cin == 2) {
       if constexpr (R >= 8)
-        if (LcdLp::matches(p.pre)) return launch_rows_fwd_b<R, 2, LcdLp>(st, p);
+        if (SlmsOnly::matches(p.pre)) return launch_rows_fwd_b<R, 2, SlmsOnly>(st, p);
       return launch_rows_fwd_b<R, 2>(st, p);
     }
     return launch_rows_fwd_b<R, 3>(st, p);
+  }
+  if (p.pol) {
+    RsLaunch q = p;
+    q.B = 2 * p.B;
+    return launch_rows_inv_b<R, 1, false, true>(st, q);
   }
   const bool epi = p.post.nops > 0 || (p.adjoint && p.cout == 3);
   if (p.cout == 1) return epi ? launch_rows_inv_b<R, 1, true>(st, p) : launch_rows_inv_b<R, 1, false>(st, p);
   return epi ? launch_rows_inv_b<R, 3, true>(st, p) : launch_rows_inv_b<R, 3, false>(st, p);
 }
 
-template <int R> int rs_blk_cols(cudaStream_t st, const RsLaunch& p) { return launch_cols_b<R>(st, p); }
+template <int R> int rs_blk_cols(cudaStream_t st, const RsLaunch& p) {
+  RsLaunch q = p;
+  if (p.pol) q.cout = 2;
+  return launch_cols_b<R>(st, q);
+}
 
 template <int R>
 int rs_blk_hhat_rows(cudaStream_t st, int ny, int nx, int py, const double* offx, const double* offy, int q2, double z,

@@ -25,6 +25,8 @@ struct RsLaunch {
   XlProg pre, post;
   int adjoint;
   int px, py;                   // points of the x and the y transform (px: columns of the intermediate)
+  int pol;                      // VRS behind a polarizer: two components, u and Ez (pre without the polarizer)
+  float pol_c, pol_s;           // cos and sin of its angle
   int lw;                       // log2 of the intermediate's column-tile width (block engine)
 };
 
