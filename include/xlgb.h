@@ -370,6 +370,14 @@ int xl_czt_transfer_plane(void* stream, int ny, int nx, const double* x, const d
 int xl_apply_ops(void* stream, int batch, int comps, int ny, int nx, const void* const* in,
                  long long in_bstride, void* const* out, long long out_bstride, const XlProg* prog);
 
+/* The program applied to a scalar field of ones (out: batch planes): the mask
+ * an SLM (optical_elements.py:87-103) or a thin lens (:678-703) returns. */
+int xl_mask_planes(void* stream, int batch, int ny, int nx, void* out, long long out_bstride, const XlProg* prog);
+
+/* The quality factor of wave_optics.py:187-191 for n distances on the device
+ * (float64): rmax the grid's largest radius, dr its pixel diagonal. */
+int xl_quality_factor(void* stream, const double* z, int n, double wavelength, double rmax, double dr, double* out);
+
 /* The per-pixel coefficients of the high-NA lens (optical_elements.py:528-594)
  * as 6 float32 planes of ny x nx: E' = K [Ex, Ey] with K = {K00, K01, K10,
  * K11, K20, K21}; they depend on the geometry only and are cached by callers. */

@@ -208,7 +208,7 @@ template <int R, int MODE> __host__ __device__ constexpr size_t rows_fwd_fixed(i
 // the bulk copies of the next row group start.  (VRS with three component groups
 // in a CTA of 768 threads and the program's results in a shared buffer between:
 // 774 us for 8 x 2048^2 behind an LCD and a polarizer, this form 467 with two
-// components; without a program 694 and WW.)  The adjoint, which has no program,
+// components; without a program 694 and 502.)  The adjoint, which has no program,
 // keeps the three groups.
 // FK: the fused program's op kinds fixed at compile time (FixedKinds<...>,
 // for the programs the benchmarks and tables run), or FixedKinds<>.

@@ -167,6 +167,15 @@ def keep_for_capture(t):
     return t
 
 
+def is_plain_cuda(t) -> bool:
+    """Whether a kernel of the library can read the tensor's memory: an ordinary
+    tensor of the current device (no subclass, no functorch transform's wrapper,
+    no lazily negated view)."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and
+            t.device.index == torch.cuda.current_device() and not t.is_neg() and
+            not torch._C._functorch.is_functorch_wrapped_tensor(t))
+
+
 _array_cache: "collections.OrderedDict" = collections.OrderedDict()
 
 
@@ -250,6 +259,12 @@ def quality_factor(x, y, wavelength, z):
     rmax = np.sqrt((x ** 2).max() + (y ** 2).max())
     if isinstance(z, torch.Tensor):
         z = z.detach().to(torch.float64)
+        if z.numel() and is_plain_cuda(z):
+            z = z.contiguous()
+            out = torch.empty_like(z)
+            _lib.check(lib().xl_quality_factor(stream_handle(), z.data_ptr(), z.numel(), float(wavelength), float(rmax),
+                                               float(dr_real), out.data_ptr()), "xl_quality_factor")
+            return out
         return (torch.sqrt(wavelength ** 2 + rmax ** 2 + 2 * wavelength * torch.sqrt(rmax ** 2 + z ** 2)) -
                 rmax) / dr_real
     z = np.asarray(z, dtype=np.float64)
@@ -376,6 +391,17 @@ def op_lens(x, y, wavelength, radius, focal, vector):
     tct = device_array(np.asarray(tc, dtype=np.float64), torch.float64)
     trt = device_array(np.asarray(tr, dtype=np.float64), torch.float64)
     return JonesOp(_lib.OP_SEPMASK, ptrs=[c, r, tct, trt], sval=[1.0 if vector else 0.0])
+
+
+def mask_planes(op, lead, ny, nx) -> torch.Tensor:
+    """The mask of one op, i.e. the op applied to a scalar field of ones, of shape lead + (ny, nx)."""
+    B = int(np.prod(lead)) if len(lead) else 1
+    out = torch.empty(tuple(lead) + (ny, nx), dtype=torch.complex64, device=device())
+    prog = _lib.XlProg()
+    fill_prog(prog, [op], ny, nx)
+    _lib.check(lib().xl_mask_planes(stream_handle(), B, ny, nx, out.data_ptr(), ny * nx, ctypes.byref(prog)),
+               "xl_mask_planes")
+    return out
 
 
 _highna_cache: "collections.OrderedDict" = collections.OrderedDict()

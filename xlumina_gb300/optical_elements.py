@@ -25,6 +25,9 @@ _VECTOR = ('Vectorized light', 'Vectorized light source')
 def _phase_mask(phase, ny, nx):
     """exp(i phase) materialised on the device (the mask an SLM returns), one
     elementwise kernel."""
+    if engine.is_plain_cuda(phase) and phase.dtype == torch.float32 and phase.dim() in (2, 3) and \
+            phase.is_contiguous() and 0 < phase.numel() < 2 ** 31 and phase.numel() <= 65535 * ny * nx:
+        return engine.mask_planes(engine.JonesOp(_lib.OP_PHASE, [phase.detach()]), phase.shape[:-2], ny, nx)
     p = phase.detach() if isinstance(phase, torch.Tensor) else torch.as_tensor(phase, device=engine.device())
     p = p.to(torch.float32)
     return torch.polar(torch.ones((), dtype=torch.float32, device=p.device).expand_as(p), p)
@@ -256,9 +259,7 @@ def lens(input_field, radius, focal):
         raise ValueError("Invalid input. Please use ScalarLight or VectorizedLight object.")
     op = engine.op_lens(input_field.x, input_field.y, input_field.wavelength, radius, focal, vector)
     ny, nx = len(input_field.y), len(input_field.x)
-    ones = torch.ones((ny, nx), dtype=torch.complex64, device=engine.device())
-    mask = engine.apply_ops([ones], [engine.op_lens(input_field.x, input_field.y, input_field.wavelength,
-                                                    radius, focal, False)], ny, nx)[0]
+    mask = engine.mask_planes(op, (), ny, nx)
     if vector:
         out = input_field._with_op(op)
         out.info = 'Vectorized light'
