@@ -45,8 +45,13 @@ def device() -> torch.device:
     return d
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle, without the Stream object that
+    ``torch.cuda.current_stream()`` builds (10 of the 105 us of a small call)."""
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _ptr(t) -> int:
@@ -113,9 +118,11 @@ def array_key(a: np.ndarray) -> bytes:
     repeated call does not copy and hash the array again."""
     k = id(a)
     hit = _bytes_keys.get(k)
-    if hit is not None and hit[0] is a:
+    if hit is not None and hit[0] is a and not a.flags.writeable:
         return hit[1]
     b = a.tobytes()
+    if a.flags.writeable or a.base is not None:
+        return b                      # its values may change: never remembered
     with _LOCK:
         _bytes_keys[k] = (a, b)       # the reference keeps the id valid
         while len(_bytes_keys) > 256:
@@ -208,16 +215,16 @@ class _Built:
 
     def __init__(self, t):
         self.t = t
-        self.stream = torch.cuda.current_stream()
+        self.stream = stream_handle()
         self.ev = torch.cuda.Event()
-        self.ev.record(self.stream)
+        self.ev.record()
 
     def use(self) -> torch.Tensor:
         if torch.cuda.is_current_stream_capturing():
             # the plan's warm-up run built it; the plan keeps it alive
             return keep_for_capture(self.t)
-        cur = torch.cuda.current_stream()
-        if cur != self.stream:
+        if stream_handle() != self.stream:
+            cur = torch.cuda.current_stream()
             if not self.ev.query():
                 cur.wait_event(self.ev)
             self.t.record_stream(cur)
@@ -250,13 +257,30 @@ def rs_wrapped_offsets(x: np.ndarray, P: int) -> np.ndarray:
     return out
 
 
+_geometry_cache: "collections.OrderedDict" = collections.OrderedDict()
+
+
+def _grid_geometry(x, y):
+    """(pixel diagonal, largest radius) of a grid, cached by its values."""
+    x, y = as_grid(x), as_grid(y)
+    key = (array_key(x), array_key(y))
+    with _LOCK:
+        g = _geometry_cache.get(key)
+        if g is not None:
+            _geometry_cache.move_to_end(key)
+            return g
+    g = (np.sqrt((x[1] - x[0]) ** 2 + (y[1] - y[0]) ** 2), np.sqrt((x ** 2).max() + (y ** 2).max()))
+    with _LOCK:
+        _geometry_cache[key] = g
+        while len(_geometry_cache) > 64:
+            _geometry_cache.popitem(last=False)
+    return g
+
+
 def quality_factor(x, y, wavelength, z):
     """wave_optics.py:187-191 / vectorized_optics.py:264-270 (a tensor distance
     gives a device tensor, computed without a host read)."""
-    dx = x[1] - x[0]
-    dy = y[1] - y[0]
-    dr_real = np.sqrt(dx ** 2 + dy ** 2)
-    rmax = np.sqrt((x ** 2).max() + (y ** 2).max())
+    dr_real, rmax = _grid_geometry(x, y)
     if isinstance(z, torch.Tensor):
         z = z.detach().to(torch.float64)
         if z.numel() and is_plain_cuda(z):
@@ -384,13 +408,32 @@ def lens_factors(x, y, wavelength, radius, focal):
     return colfac, rowfac, x ** 2 / rx ** 2, y ** 2 / ry ** 2
 
 
+_lens_cache: "collections.OrderedDict" = collections.OrderedDict()
+
+
 def op_lens(x, y, wavelength, radius, focal, vector):
-    colfac, rowfac, tc, tr = lens_factors(x, y, wavelength, radius, focal)
-    c = device_array(colfac.astype(np.complex64), torch.complex64)
-    r = device_array(rowfac.astype(np.complex64), torch.complex64)
-    tct = device_array(np.asarray(tc, dtype=np.float64), torch.float64)
-    trt = device_array(np.asarray(tr, dtype=np.float64), torch.float64)
-    return JonesOp(_lib.OP_SEPMASK, ptrs=[c, r, tct, trt], sval=[1.0 if vector else 0.0])
+    """The thin lens as a separable mask; its factors on the device are cached by geometry."""
+    x, y = as_grid(x), as_grid(y)
+    numbers = (wavelength, *radius, *focal)
+    key = ptrs = None
+    if all(isinstance(v, (int, float)) for v in numbers):
+        key = (array_key(x), array_key(y), numbers, len(radius), torch.cuda.current_device())
+        with _LOCK:
+            ptrs = _lens_cache.get(key)
+            if ptrs is not None:
+                _lens_cache.move_to_end(key)
+    if ptrs is None:
+        colfac, rowfac, tc, tr = lens_factors(x, y, wavelength, radius, focal)
+        ptrs = (device_array(colfac.astype(np.complex64), torch.complex64),
+                device_array(rowfac.astype(np.complex64), torch.complex64),
+                device_array(np.asarray(tc, dtype=np.float64), torch.float64),
+                device_array(np.asarray(tr, dtype=np.float64), torch.float64))
+        if key is not None:
+            with _LOCK:
+                _lens_cache[key] = ptrs
+                while len(_lens_cache) > 64:
+                    _lens_cache.popitem(last=False)
+    return JonesOp(_lib.OP_SEPMASK, ptrs=[keep_for_capture(t) for t in ptrs], sval=[1.0 if vector else 0.0])
 
 
 def mask_planes(op, lead, ny, nx) -> torch.Tensor:
@@ -670,7 +713,10 @@ class RsCall:
                 spec_index = device_array(np.arange(B, dtype=np.int32), torch.int32)
             zt = (zd if zd.numel() == B else zd.expand(B).contiguous()) if vector else None
         else:
-            zs = [float(v) for v in np.broadcast_to(np.asarray(z, dtype=np.float64), (B,))]
+            if isinstance(z, (int, float)):
+                zs = [float(z)] * B
+            else:
+                zs = [float(v) for v in np.broadcast_to(np.asarray(z, dtype=np.float64), (B,))]
             uniq = sorted(set(zs))
             specs = [SPECTRA.get(x, y, zz, wavelength, dz) for zz in uniq]
             if len(specs) == 1:
@@ -680,6 +726,7 @@ class RsCall:
                 spec_ptrs = device_array([specs[uniq.index(v)].data_ptr() for v in zs], torch.int64)
             zt = device_array(np.asarray(zs, dtype=np.float64), torch.float64) if vector else None
         cout = 3 if vector else 1
+        given = outs is not None
         if work is None:
             work = torch.empty(L.xl_rs_work_bytes(B, cout, ny, nx) // 8, dtype=torch.complex64, device=dev)
         if outs is None:
@@ -693,7 +740,7 @@ class RsCall:
         for i, c in enumerate(comps):
             a.inp[i] = c.data_ptr()
         for i, o in enumerate(outs):
-            a.out[i] = out_pointer(o, tuple(lead) + (ny, nx))
+            a.out[i] = out_pointer(o, tuple(lead) + (ny, nx)) if given else o.data_ptr()
         a.in_bstride = ibs
         a.out_bstride = ny * nx
         if vector:
@@ -788,7 +835,7 @@ def bluestein_length(m, M):
     if M < 2:
         raise ValueError("chirp-z needs at least 2 output samples per axis")
     mp = m + M - 1
-    L = int(2 ** int(np.ceil(np.log2(mp))))
+    L = 1 << (mp - 1).bit_length()
     if L == mp:
         raise ValueError(f"m + M - 1 = {mp} is a power of two: the reference's Bluestein output slice "
                          "(wave_optics.py:446) is one sample short for this size")
