@@ -377,17 +377,6 @@ __device__ __forceinline__ void apply_prog_fixed(const XlProg& prog, float2 (&e)
   }
 }
 
-// The same for one pixel.
-template <class FK, int K = 0, class PR>
-__device__ __forceinline__ void apply_prog_fixed1(const XlProg& prog, float2 (&e)[3], const PixelCtx& px,
-                                                  const PR& pr) {
-  static_assert(FK::n > 0 && FK::n <= XL_MAX_OPS, "a fixed program");
-  if constexpr (K < FK::n) {
-    apply_kind<FK::at(K)>(prog.ops[K], K, e, px, pr);
-    apply_prog_fixed1<FK, K + 1>(prog, e, px, pr);
-  }
-}
-
 template <class PR>
 __device__ __forceinline__ void apply_prog_r(const XlProg& prog, float2 (&e)[3], const PixelCtx& px, const PR& pr) {
   for (int i = 0; i < prog.nops; ++i) apply_op_r(prog.ops[i], i, e, px, pr);

@@ -1,8 +1,9 @@
 // Rayleigh-Sommerfeld propagation (scalar RS and vectorial VRS): the C ABI
 // entry points.  The reference (wave_optics.py:281-289) zero-pads the N x N
 // field to (2N-1)^2, multiplies fft2(U) by fft2(H) and crops [N-1:, N-1:];
-// the kernels (rs_kernels.cuh) run the same linear convolution on a 2Q x 2Q
-// grid, Q the next power of two >= N, in three passes.
+// the kernels run the same linear convolution on a grid that holds it, in three
+// passes: up to 256 pixels a side on the Stockham engine (rs_kernels.cuh), above
+// on the block engine (rs_blk.cuh), axes above 2048 in two halves (rs_half.cuh).
 #include <math.h>
 
 #include <mutex>
@@ -11,26 +12,30 @@
 
 namespace xl {
 
-// CALL(LOGQ) for the Stockham engine's lengths, CALL(R) for the block engine's.
+// CALL(LOGQ) for the Stockham engine's lengths.
 #define XL_RS_DISPATCH(LOGQ_VAR, CALL)          \
   switch (LOGQ_VAR) {                           \
     case 5: return CALL(5);                     \
     case 6: return CALL(6);                     \
     case 7: return CALL(7);                     \
     case 8: return CALL(8);                     \
-    case 12: return CALL(12);                   \
     default: break;                             \
   }
-#define XL_RS_BLK_DISPATCH(R_VAR, CALL)         \
-  switch (R_VAR) {                              \
-    case 4: return CALL(4);                     \
-    case 6: return CALL(6);                     \
-    case 8: return CALL(8);                     \
-    case 10: return CALL(10);                   \
-    case 12: return CALL(12);                   \
-    case 14: return CALL(14);                   \
-    case 16: return CALL(16);                   \
-    default: break;                             \
+// NAME<R>(args) of an axis of P points: 256 R, or two halves of 256 R.
+#define XL_RS_BLK_DISPATCH(P, NAME, ...)                      \
+  switch (P) {                                                \
+    case 1024: return rs_blk_##NAME<4>(__VA_ARGS__);          \
+    case 1536: return rs_blk_##NAME<6>(__VA_ARGS__);          \
+    case 2048: return rs_blk_##NAME<8>(__VA_ARGS__);          \
+    case 2560: return rs_blk_##NAME<10>(__VA_ARGS__);         \
+    case 3072: return rs_blk_##NAME<12>(__VA_ARGS__);         \
+    case 3584: return rs_blk_##NAME<14>(__VA_ARGS__);         \
+    case 4096: return rs_blk_##NAME<16>(__VA_ARGS__);         \
+    case 5120: return rs_half_##NAME<10>(__VA_ARGS__);        \
+    case 6144: return rs_half_##NAME<12>(__VA_ARGS__);        \
+    case 7168: return rs_half_##NAME<14>(__VA_ARGS__);        \
+    case 8192: return rs_half_##NAME<16>(__VA_ARGS__);        \
+    default: break;                                           \
   }
 
 static int unsupported(const char* what) {
@@ -38,25 +43,20 @@ static int unsupported(const char* what) {
   return XL_EUNSUPPORTED;
 }
 
-static int blk_rows(int r, cudaStream_t st, const RsLaunch& p, bool inverse) {
-#define CALL(R) rs_blk_rows<R>(st, p, inverse)
-  XL_RS_BLK_DISPATCH(r, CALL)
-#undef CALL
+static int blk_rows(cudaStream_t st, const RsLaunch& p, bool inverse) {
+  XL_RS_BLK_DISPATCH(p.px, rows, st, p, inverse)
   return unsupported("xl_rs_propagate");
 }
 
-static int blk_cols(int r, cudaStream_t st, const RsLaunch& p) {
-#define CALL(R) rs_blk_cols<R>(st, p)
-  XL_RS_BLK_DISPATCH(r, CALL)
-#undef CALL
+static int blk_cols(cudaStream_t st, const RsLaunch& p) {
+  XL_RS_BLK_DISPATCH(p.py, cols, st, p)
   return unsupported("xl_rs_propagate");
 }
 
 static int blk_propagate(cudaStream_t st, const RsLaunch& p, int stage) {
-  const int rx = p.px / 256, ry = p.py / 256;
   for (int s = 0; s < 3; ++s) {
     if (stage >= 0 && s != stage) continue;
-    if (int rc = s == 1 ? blk_cols(ry, st, p) : blk_rows(rx, st, p, s == 2)) return rc;
+    if (int rc = s == 1 ? blk_cols(st, p) : blk_rows(st, p, s == 2)) return rc;
   }
   return XL_OK;
 }
@@ -75,21 +75,17 @@ static int spectrum(cudaStream_t st, int ny, int nx, const double* offx, const d
   const int lq = rs_logq(ny, nx);
   if (rs_is_blk(ny, nx)) {
     const int px = rs_px(ny, nx), py = rs_py(ny, nx), q2 = 2 << lq;
-    auto rows = [&](int r) {
-#define CALL(R) rs_blk_hhat_rows<R>(st, ny, nx, py, offx, offy, q2, z, zp, wavelength, dz, spec, work)
-      XL_RS_BLK_DISPATCH(r, CALL)
-#undef CALL
+    auto rows = [&]() {
+      XL_RS_BLK_DISPATCH(px, hhat_rows, st, ny, nx, py, offx, offy, q2, z, zp, wavelength, dz, spec, work)
       return unsupported("xl_rs_transfer_spectrum");
     };
     const float sc = (float)(scale * ((double)q2 * q2 / ((double)px * py)));
-    auto cols = [&](int r) {
-#define CALL(R) rs_blk_hhat_cols<R>(st, work, px, sc, spec)
-      XL_RS_BLK_DISPATCH(r, CALL)
-#undef CALL
+    auto cols = [&]() {
+      XL_RS_BLK_DISPATCH(py, hhat_cols, st, work, px, sc, spec)
       return unsupported("xl_rs_transfer_spectrum");
     };
-    if (int rc = rows(px / 256)) return rc;
-    return cols(py / 256);
+    if (int rc = rows()) return rc;
+    return cols();
   }
 #define CALL(L) rs_spectrum<L>(st, ny, nx, offx, offy, z, zp, wavelength, scale, spec, work, dz)
   XL_RS_DISPATCH(lq, CALL)
@@ -231,7 +227,8 @@ static int rs_run(void* stream, const XlRsArgs* a, int stage) {
   // its Ex and Ey are c and s times one field, and so are their propagations,
   // so two components are transformed instead of three.
   p.pol = 0;
-  if (vector && !a->adjoint && a->pre.nops > 0 && a->post.nops == 0 && rs_is_blk(a->ny, a->nx)) {
+  if (vector && !a->adjoint && a->pre.nops > 0 && a->post.nops == 0 && rs_is_blk(a->ny, a->nx) &&
+      !rs_is_half(a->nx)) {
     const XlOp& lp = a->pre.ops[a->pre.nops - 1];
     if (lp.kind == XL_OP_LP && !(lp.pmask & 1)) {
       p.pol = 1;

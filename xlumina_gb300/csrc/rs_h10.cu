@@ -1,0 +1,5 @@
+// RS / VRS passes of 5120-point transforms as two halves (one translation unit of
+// rs_half.cuh).
+#include "rs_half.cuh"
+
+XL_RS_HALF_INSTANTIATE(10)

@@ -53,10 +53,8 @@ template <int LOGQ> struct RsCfg {
   static constexpr int XS = P + P / 16;                       // exchange slots per line
   static constexpr int G = (256 / T) > 1 ? (256 / T) : 1;     // lines per CTA in the row passes
   static constexpr int ROW_THREADS = G * T;
-  // Column-tile width of the intermediate and spectrum layouts.  At Q = 2048
-  // the tiles are 8 columns wide, so a warp's row access is four 64-byte
-  // pieces; the column pass takes half a tile per CTA.
-  static constexpr int W = LOGQ >= 12 ? 2 : ((32 / T) > 4 ? (32 / T) : 4);
+  // Column-tile width of the intermediate and spectrum layouts.
+  static constexpr int W = (32 / T) > 4 ? (32 / T) : 4;
   // Column-pass (and spectrum-build) CTAs take CW columns of a tile,
   // interleaved in the lanes of every warp.
   static constexpr int CW = W;
@@ -180,9 +178,7 @@ template <int LOGQ, int NC> struct RowCfg {
 // prologue runs the fused program over every pixel and writes the components
 // to a shared buffer; the stage is then free, so the bulk copies of the next
 // row group start while the component groups transform this one.
-// FK: the fused program's op kinds fixed at compile time (FixedKinds<...>,
-// for the programs the benchmarks and tables run), or FixedKinds<>.
-template <int LOGQ, int MODE, class FK = FixedKinds<>>
+template <int LOGQ, int MODE>
 __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowCfg<LOGQ, MODE == 1 ? 1 : 3>::MINB)
     rs_rows_fwd(const __grid_constant__ RsLaunch p, const __grid_constant__ RowStage st) {
   using C = RsCfg<LOGQ>;
@@ -235,7 +231,7 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
       int last = -1;
       float Y = 0.f, z2 = 0.f;
       for (int idx = tid; idx < C::G * nx; idx += F::THREADS) {
-        const int g2 = C::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, r = r0 + g2;
+        const int g2 = idx / nx, n = idx - g2 * nx, r = r0 + g2;
         if (r >= ny) break;
         const long long pix = (long long)r * nx + n;
         float2 e[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -244,9 +240,7 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
           const int fo = st.fld[c];
           e[c] = fo >= 0 ? ((const float2*)(stage + fo))[g2 * nx + n] : p.in[c][(long long)b * p.ibs + pix];
         }
-        if constexpr (FK::n > 0) {
-          apply_prog_fixed1<FK>(p.pre, e, PixelCtx{r, n, pix, b}, StagedParams{stage, &st, g2, nx, n});
-        } else if (p.pre.nops) {
+        if (p.pre.nops) {
           PixelCtx px{r, n, pix, b};
           apply_prog_r(p.pre, e, px, StagedParams{stage, &st, g2, nx, n});
         }
@@ -265,16 +259,11 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
         for (int c = 0; c < NC; ++c) post[(c * C::G + g2) * nx + n] = e[c];
       }
     } else
-    // CTAs of up to 256 threads: four pixels per thread at a time while four
+    // CTAs of 256 threads (scalar RS): four pixels per thread at a time while four
     // remain, then one; each op of the program is dispatched once for the
     // four, and their loads and arithmetic overlap
     {
       const int lim = min(C::G, ny - r0) * nx;
-      const float zb = MODE == 2 ? (float)p.z[b] : 0.f;
-      // one row per group (every 2048-point line and longer): its y and
-      // y^2 + z^2 once for the group instead of once per pixel
-      const float Y0 = MODE == 2 && C::G == 1 ? (float)p.y[r0] : 0.f;
-      const float z20 = Y0 * Y0 + zb * zb;
       auto chunk = [&](auto npx, int base) {
         constexpr int NPX = decltype(npx)::value;
         float2 e[NPX][3];
@@ -283,7 +272,7 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
 #pragma unroll
         for (int q = 0; q < NPX; ++q) {
           const int idx = base + q * F::THREADS;
-          const int g2 = C::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, r = r0 + g2;
+          const int g2 = idx / nx, n = idx - g2 * nx, r = r0 + g2;
           const long long pix = (long long)r * nx + n;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -296,18 +285,10 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, MODE == 1 ? 1 : 3>::THREADS, RowC
           px[q] = PixelCtx{r, n, pix, b};
           pr[q] = StagedParams{stage, &st, g2, nx, n};
         }
-        if constexpr (FK::n > 0) apply_prog_fixed<FK>(p.pre, e, px, pr);
-        else if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
+        if (p.pre.nops) apply_prog_vec<NPX>(p.pre, e, px, pr);
 #pragma unroll
         for (int q = 0; q < NPX; ++q) {
           const int r = px[q].row, n = px[q].col;
-          if constexpr (MODE == 2) {  // vectorized_optics.py:258-261, Ez = Ex X/r + Ey Y/r
-            const float Y = C::G == 1 ? Y0 : (float)p.y[r];
-            const float z2 = C::G == 1 ? z20 : Y * Y + zb * zb;
-            const float X = xf[n];
-            const float inv = rsqrtf(X * X + z2);
-            e[q][2] = cadd(cscale(e[q][0], X * inv), cscale(e[q][1], Y * inv));
-          }
 #pragma unroll
           for (int c = 0; c < NC; ++c) post[(c * C::G + (r - r0)) * nx + n] = e[q][c];
         }
@@ -498,7 +479,7 @@ __global__ void __launch_bounds__(RowCfg<LOGQ, COUT>::THREADS, RowCfg<LOGQ, COUT
       int last = -1;
       float Y = 0.f, z2 = 0.f;
       for (int idx = tid; idx < C::G * nx; idx += F::THREADS) {
-        const int g2 = C::G == 1 ? 0 : idx / nx, n = idx - g2 * nx, ro = r0 + g2;
+        const int g2 = idx / nx, n = idx - g2 * nx, ro = r0 + g2;
         if (ro >= ny) break;
         const long long o = (long long)b * p.obs + (long long)ro * nx + n;
         float2 e[3];
@@ -557,7 +538,7 @@ int rs_spectrum(cudaStream_t st, int ny, int nx, const double* offx, const doubl
   return XL_OK;
 }
 
-template <int LOGQ, int MODE, class FK = FixedKinds<>>
+template <int LOGQ, int MODE>
 static int launch_rows_fwd(cudaStream_t s, const RsLaunch& p) {
   using C = RsCfg<LOGQ>;
   constexpr int NC = MODE == 1 ? 1 : 3;
@@ -572,10 +553,10 @@ static int launch_rows_fwd(cudaStream_t s, const RsLaunch& p) {
     return XL_EUNSUPPORTED;
   }
   int per_sm;
-  if (int rc = launch_ready<rs_rows_fwd<LOGQ, MODE, FK>>(F::THREADS, sm, &per_sm, "rs_rows_fwd")) return rc;
+  if (int rc = launch_ready<rs_rows_fwd<LOGQ, MODE>>(F::THREADS, sm, &per_sm, "rs_rows_fwd")) return rc;
   const int total = p.B * ((p.ny + C::G - 1) / C::G);
   const int grid = persistent_grid(per_sm, total);
-  rs_rows_fwd<LOGQ, MODE, FK><<<grid, F::THREADS, sm, s>>>(p, st);
+  rs_rows_fwd<LOGQ, MODE><<<grid, F::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("rs_rows_fwd");
   return XL_OK;
 }
@@ -613,21 +594,8 @@ template <int LOGQ>
 static int launch_stage(cudaStream_t st, const RsLaunch& p, int stage) {
   using C = RsCfg<LOGQ>;
   if (stage == 0) {
-    // the programs of the benchmarks' fields (1024^2 and larger) get a kernel
-    // with their op kinds fixed: a phase SLM before scalar RS, an LCD and a
-    // polarizer before VRS
-    using SlmOnly = FixedKinds<XL_OP_PHASE>;
-    using LcdLp = FixedKinds<XL_OP_LCD, XL_OP_LP>;
-    if (p.cout == 1) {
-      if constexpr (LOGQ >= 10)
-        if (SlmOnly::matches(p.pre)) return launch_rows_fwd<LOGQ, 1, SlmOnly>(st, p);
-      return launch_rows_fwd<LOGQ, 1>(st, p);
-    }
-    if (p.cin == 2) {
-      if constexpr (LOGQ >= 10)
-        if (LcdLp::matches(p.pre)) return launch_rows_fwd<LOGQ, 2, LcdLp>(st, p);
-      return launch_rows_fwd<LOGQ, 2>(st, p);
-    }
+    if (p.cout == 1) return launch_rows_fwd<LOGQ, 1>(st, p);
+    if (p.cin == 2) return launch_rows_fwd<LOGQ, 2>(st, p);
     return launch_rows_fwd<LOGQ, 3>(st, p);
   } else if (stage == 1) {
     return launch_cols<LOGQ>(st, p);
