@@ -451,6 +451,15 @@ int xl_beam_splitter_backward(void* stream, const XlBsArgs* args, const void* co
 int xl_re_inner(void* stream, int planes, long long npix, const void* a, long long a_pstride, const void* b,
                 long long b_pstride, void* work, void* out);
 
+/* The intensity MSE (loss_functions.py:93-107) of three components, each a
+ * tensor of `planes` planes, in one launch: out[3][planes]; work as for 3 planes
+ * times `planes`.  The gradients of components whose ga and gb are NULL are left out. */
+int xl_vmse_intensity(void* stream, int planes, long long npix, const void* const* a, long long a_pstride,
+                      const void* const* b, long long b_pstride, void* work, void* out);
+int xl_vmse_intensity_grad(void* stream, int planes, long long npix, const void* const* a, long long a_pstride,
+                           const void* const* b, long long b_pstride, const void* gloss, void* const* ga,
+                           void* const* gb);
+
 /* Per-plane MSE of kind 0 intensity (= xl_mse_intensity), 1 amplitude
  * sum (|a| - |b|)^2 / npix (MSE_Amplitude, loss_functions.py:109-121) or
  * 2 phase sum (arg a - arg b)^2 / npix (MSE_Phase, :123-135; vMSE_* at

@@ -175,6 +175,14 @@ SIGNATURES = {
     "xl_mse_intensity_grad": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p,
                                              ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong,
                                              ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
+    "xl_vmse_intensity": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong,
+                                         ctypes.POINTER(ctypes.c_void_p), ctypes.c_longlong,
+                                         ctypes.POINTER(ctypes.c_void_p), ctypes.c_longlong, ctypes.c_void_p,
+                                         ctypes.c_void_p]),
+    "xl_vmse_intensity_grad": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong,
+                                              ctypes.POINTER(ctypes.c_void_p), ctypes.c_longlong,
+                                              ctypes.POINTER(ctypes.c_void_p), ctypes.c_longlong, ctypes.c_void_p,
+                                              ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p)]),
     "xl_plane_mse": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p,
                                     ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p,
                                     ctypes.c_void_p]),

@@ -223,6 +223,29 @@ def mse_intensity(a, b, kind="intensity"):
     return _MseIntensity.apply(a, b, kind)
 
 
+class _VMseIntensity(torch.autograd.Function):
+    """Intensity MSE of a vector field's three components, one launch each way."""
+
+    @staticmethod
+    def forward(ctx, *fields):
+        ctx.save_for_backward(*fields)
+        return engine.vmse_intensity(fields[:3], fields[3:])
+
+    @staticmethod
+    def backward(ctx, g):
+        f = ctx.saved_tensors
+        grads = engine.vmse_intensity_grad(f[:3], f[3:], g, ctx.needs_input_grad)
+        return tuple(d if d is None or d.shape == t.shape else d.reshape((-1,) + tuple(t.shape)).sum(0)
+                     for d, t in zip(grads, f))
+
+
+def vmse_intensity(a, b):
+    """Intensity MSE of the components a = (Ex, Ey, Ez) against b, stacked."""
+    if all(isinstance(t, torch.Tensor) for t in (*a, *b)) and engine.vmse_shapes(a, b):
+        return _VMseIntensity.apply(*a, *b)
+    return torch.stack([mse_intensity(p, q) for p, q in zip(a, b)])
+
+
 class _AreaLoss(torch.autograd.Function):
     """small_area_hybrid per plane (fused passes of libxlgb) with the
     hand-written gradient seeded per plane."""

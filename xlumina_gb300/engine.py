@@ -1226,6 +1226,45 @@ def mse_intensity_grad(a, b, g, want_a=True, want_b=False, kind: str = "intensit
     return ga, gb
 
 
+def vmse_shapes(a, b) -> bool:
+    """Whether one launch takes the three components a and targets b: ordinary contiguous
+    complex64 tensors on the device, all a of one shape, all b of one shape, b like a or one plane."""
+    sa, sb = a[0].shape, b[0].shape
+    if not all(is_plain_cuda(t) and t.dtype == torch.complex64 and t.is_contiguous() and not t.is_conj() and t.numel()
+               for t in (*a, *b)) or any(t.shape != sa for t in a) or any(t.shape != sb for t in b):
+        return False
+    return len(sa) >= 2 and sb[-2:] == sa[-2:] and (sb == sa or len(sb) == 2) and \
+        a[0].numel() <= 65535 * sa[-2] * sa[-1]
+
+
+def _ptr3(ts):
+    return (ctypes.c_void_p * 3)(*[_ptr(t) for t in ts])
+
+
+def vmse_intensity(a, b) -> torch.Tensor:
+    """``mse_intensity`` of three components (``vmse_shapes``), stacked."""
+    npix = a[0].shape[-2] * a[0].shape[-1]
+    n = a[0].numel() // npix
+    L = lib()
+    work = torch.empty(max(1, L.xl_mse_intensity_work_bytes(3 * n, npix) // 8), dtype=torch.float64, device=a[0].device)
+    out = torch.empty((3,) + tuple(a[0].shape[:-2]), dtype=torch.float32, device=a[0].device)
+    _lib.check(L.xl_vmse_intensity(stream_handle(), n, npix, _ptr3(a), npix, _ptr3(b),
+                                   npix if b[0].shape == a[0].shape else 0, work.data_ptr(), out.data_ptr()),
+               "xl_vmse_intensity")
+    return out
+
+
+def vmse_intensity_grad(a, b, g, want):
+    """Gradients (shaped as a) of ``vmse_intensity`` for the wanted ones of the six tensors."""
+    npix = a[0].shape[-2] * a[0].shape[-1]
+    g = g.to(device=a[0].device, dtype=torch.float32).contiguous()
+    grads = [torch.empty_like(a[0]) if w else None for w in want]
+    _lib.check(lib().xl_vmse_intensity_grad(stream_handle(), a[0].numel() // npix, npix, _ptr3(a), npix, _ptr3(b),
+                                            npix if b[0].shape == a[0].shape else 0, g.data_ptr(), _ptr3(grads[:3]),
+                                            _ptr3(grads[3:])), "xl_vmse_intensity_grad")
+    return grads
+
+
 def z_values(z):
     """(the distance as the propagators take it, the tensor that needs its
     gradient or None).  A tensor distance stays on the device: its transfer

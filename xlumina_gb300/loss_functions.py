@@ -95,5 +95,5 @@ def vMSE_Phase(input_light, target_light):
 def vMSE_Intensity(input_light, target_light):
     """loss_functions.py:93-107: MSE_Intensity of each of Ex, Ey, Ez (stacked
     results, leading dimension 3), without stacking the fields themselves."""
-    return torch.stack([MSE_Intensity(getattr(input_light, c), getattr(target_light, c))
-                        for c in ("Ex", "Ey", "Ez")])
+    return autograd.vmse_intensity((input_light.Ex, input_light.Ey, input_light.Ez),
+                                   (target_light.Ex, target_light.Ey, target_light.Ez))
