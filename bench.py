@@ -143,17 +143,16 @@ class ClockSampler:
 # launch (4 distances, so pairs of fields share a transfer spectrum) with
 # NCU_TRAFFIC_COMMAND below; the row passes' from a batch-2 capture (--batch 2)
 # scaled per field (every field is an independent slice of those launches).
-# The column-pass variants move the same bytes (within 2 % at batch 2).
-NCU_TRAFFIC_PER_FIELD = {"rs_rows_fwd": 276.15e6, "rs_cols_conv": 478.88e6, "rs_rows_inv": 283.60e6}
-# Warp instructions per 2048^2 VRS field of the column pass, by kernel variant
-# (ncu smsp__inst_executed.sum of one launch of the batch-2 case, halved; the
-# instruction stream does not depend on the batch): NCU_INST_COMMAND below
-# with V = 8 and 10.  The pass's issue ceiling is 4 warp instructions per
-# cycle per SM (one per scheduler).
-NCU_COL_INST_PER_FIELD = {8: 303.87e6 / 2, 10: 314.38e6 / 2}
+NCU_TRAFFIC_PER_FIELD = {"rs_rows_fwd_b": 209.7e6, "rs_cols_b": 329.2e6, "rs_rows_inv_b": 214.4e6}
+# Warp instructions per 2048^2 VRS field of the column pass (ncu
+# smsp__inst_executed.sum of one launch of the batch-2 case, halved; the
+# instruction stream does not depend on the batch): NCU_INST_COMMAND below.
+# The pass's issue ceiling is 4 warp instructions per cycle per SM (one per
+# scheduler).
+NCU_COL_INST_PER_FIELD = 211.65e6 / 2
 NCU_INST_COMMAND = ("ncu --metrics smsp__inst_executed.sum --clock-control none -k regex:rs_cols -s 4 -c 1 "
                     "python bench.py --steps 2 --warmup 3 --batch 2 --no-cpu-baseline --no-fwd-bwd --no-serving "
-                    "--no-parity --col-variant V")
+                    "--no-parity --col-variant 0")
 NCU_TRAFFIC_COMMAND = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum "
                        "--clock-control none -k regex:rs_cols -s 1 -c 1 python bench.py --steps 10 --warmup 3 "
                        "--no-cpu-baseline --no-fwd-bwd --no-serving")
@@ -383,8 +382,9 @@ def run_gpu(args):
 
     # roofline: algorithmic bytes per launch (B fields), per stage
     n2 = N * N
-    alg = [72 * n2 * B, 128 * n2 * B, 72 * n2 * B]
-    names = ["rs_rows_fwd", "rs_cols_conv", "rs_rows_inv"]
+    # (behind the polarizer two components are transformed: u and Ez)
+    alg = [56 * n2 * B, 96 * n2 * B, 56 * n2 * B]
+    names = ["rs_rows_fwd_b", "rs_cols_b", "rs_rows_inv_b"]
     dom = int(np.argmax(stage_ms))
     peaks = {}
     try:
@@ -475,13 +475,13 @@ def run_gpu(args):
     # per launch (ncu, per variant) over the SMs' issue rate at the SM clock
     # sampled while the timed region ran
     clocks = clk.summary()
-    inst = NCU_COL_INST_PER_FIELD.get(int(tuned["variant"]))
+    inst = NCU_COL_INST_PER_FIELD
     issue_roofline = None
-    if inst is not None and clocks.get("sm_mhz"):
+    if clocks.get("sm_mhz"):
         n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
         ipeak = n_sm * 4 * float(clocks["sm_mhz"]) * 1e6
         iach = inst * B / (stage_ms[1] / 1e3)
-        issue_roofline = {"bound": "instruction issue", "kernel": "rs_cols_conv", "variant": int(tuned["variant"]),
+        issue_roofline = {"bound": "instruction issue", "kernel": "rs_cols_b", "variant": int(tuned["variant"]),
                           "achieved": iach, "peak": ipeak, "unit": "warp instructions/s", "frac": iach / ipeak,
                           "instructions_per_launch": inst * B,
                           "source": "ncu smsp__inst_executed.sum per field x fields per launch: " + NCU_INST_COMMAND,
@@ -513,17 +513,9 @@ def run_gpu(args):
         "stages_ms": dict(zip(names, stage_ms)),
         "column_pass_variant": {"chosen": tuned["variant"], "transform_length": 1 << col_logp,
                                 "ms_per_launch": {str(k): v for k, v in tuned["ms"].items()},
-                                "variants": "0 one line per thread; 1 two lines per thread (packed FP32), "
-                                            "pairs interleaved in warps; 2 packed, pairs in barrier groups; "
-                                            "3 one line per thread with L2 prefetch; 4 packed interleaved "
-                                            "with L2 and register prefetch; 5 one line per thread, two "
-                                            "barrier groups; 6 one line per thread, two CTAs per SM; 7 as 5 with "
-                                            "the groups started half a component apart; 8 one line per thread, "
-                                            "persistent (the library's default at 4096 points); 9 (4096 "
-                                            "points) radix-64, 64 elements per thread, one exchange per "
-                                            "transform; 10 (4096 points) as 8, each unit's spectrum values "
-                                            "kept in Tensor Memory for its second and third components"},
-        "pipeline_roofline": {"alg_bytes_per_field": 272 * n2, "achieved": pipe_gbs, "frac": pipe_gbs / peak},
+                                "variants": "one kernel per transform length (block engine), which every "
+                                            "number selects"},
+        "pipeline_roofline": {"alg_bytes_per_field": 208 * n2, "achieved": pipe_gbs, "frac": pipe_gbs / peak},
         "plain_path": {"value": plain, "unit": "fields/s", "how": "one VRS_propagation call per field"},
         "e2e": {"value": e2e, "unit": "fields/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "segments": segments, "steps_per_segment": ke,

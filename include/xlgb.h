@@ -169,8 +169,8 @@ int xl_rs_transfer_spectra_device_z(void* stream, int ny, int nx, const double* 
 
 /* Bytes of one transfer spectrum for an ny x nx field: at most (2Q)^2
  * complex64, Q = next power of two >= max(ny, nx).  Fields with a longer side
- * of 257 to 2048 take, for each axis, the shortest transform of 512 k points
- * (k = 2..8) that holds it. */
+ * above 256 take, for each axis, the shortest transform that holds it: 512 k
+ * points (k = 2..8) up to 2048 pixels, 1024 k (k = 5..8) above. */
 size_t xl_rs_spectrum_bytes(int ny, int nx);
 /* Bytes of workspace xl_rs_transfer_spectrum needs. */
 size_t xl_rs_spectrum_work_bytes(int ny, int nx);

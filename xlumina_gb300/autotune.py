@@ -127,9 +127,9 @@ class VariantTuner:
     """Kernel variant of a pass chosen by measurement, per GPU model.
 
     The library has several kernels for some passes at one transform length
-    (the one-line column pass and the packed two-line ones, interleaved in
-    the warps or in barrier groups); they agree to float32 rounding and differ
-    in speed by GPU and workload shape.  ``best_variant(pass_id, log2_len,
+    (chirp-z at the Stockham lengths: how much is staged, registers for one or
+    two CTAs per SM, persistent or not); they agree to float32 rounding and
+    differ in speed by GPU and workload shape.  ``best_variant(pass_id, log2_len,
     measure)`` times every variant with ``measure()`` (seconds of one launch,
     device work included) and selects the fastest in the library
     (``xl_set_kernel_variant``); the choice is cached with the batch packings,
