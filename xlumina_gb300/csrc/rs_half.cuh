@@ -10,8 +10,8 @@
 // over the other half (a column's input, then its first half's output) stays in
 // the thread's own Tensor Memory cells.
 //
-// 8192-point Stockham transforms, this form: 2 x 4096^2 scalar RS 1809 us, 1140;
-// one 4096^2 VRS 2513, 1587.  Shorter lengths: 4 x 2500^2 2979, 972 (5120 points);
+// 8192-point Stockham transforms, this form: 2 x 4096^2 scalar RS 1809 us, 1088;
+// one 4096^2 VRS 2513, 1542.  Shorter lengths: 4 x 2500^2 2979, 930 (5120 points);
 // 4 x 300 x 4096 1797, 222 (1024 points in y).
 #pragma once
 
@@ -196,11 +196,14 @@ template <int R> struct HalfRow {
 // row's elements after the program stay in shared memory for both halves; the
 // phase A twiddles and w_P^n of the thread's elements are in Tensor Memory.
 //
-// What bounds it: the row's loads are not overlapped with its transform within a
-// group (2 x 4096^2 scalar behind an SLM: 319 us at 2.5 TB/s; Stockham 501); a
-// row staged ahead by bulk copies does not fit beside three lines and rows.
+// A row's loads are not overlapped with its transform within a group, and a row
+// staged ahead by bulk copies does not fit beside three lines and rows, so a
+// group's next rows are prefetched into L2 while it transforms (where bulk
+// prefetches may read them: 16-byte aligned planes and rows).  2 x 4096^2 scalar
+// behind an SLM: 320 us without, 264 with (3.6 TB/s; Stockham 501); one 4096^2 VRS
+// 359, 313.
 template <int R, int MODE, class FK = FixedKinds<>>
-__global__ void __launch_bounds__(HalfRow<R>::THREADS, 1) rs_rows_fwd_h(const __grid_constant__ RsLaunch p) {
+__global__ void __launch_bounds__(HalfRow<R>::THREADS, 1) rs_rows_fwd_h(const __grid_constant__ RsLaunch p, const __grid_constant__ RowStage st) {
   using F = BlkFft<R>;
   constexpr int M = F::P, THREADS = HalfRow<R>::THREADS;
   constexpr bool ONE = MODE == 1;
@@ -274,6 +277,7 @@ __global__ void __launch_bounds__(HalfRow<R>::THREADS, 1) rs_rows_fwd_h(const __
         }
       }
     }
+    if (lane0 == 0 && u + step < total) prefetch_rows(st, (u + step) % p.B, (u + step) / p.B, 1);
     if constexpr (ONE) sync();
     else __syncthreads();
     const int plane = ONE ? b : b * COUT + cg;
@@ -491,7 +495,9 @@ template <int R, int MODE, class FK = FixedKinds<>> static int launch_rows_fwd_h
   int per_sm;
   if (int rc = launch_ready<rs_rows_fwd_h<R, MODE, FK>>(K::THREADS, sm, &per_sm, "rs_rows_fwd_h")) return rc;
   const int total = p.B * p.ny, units = MODE == 1 ? (total + 2) / 3 : total;
-  rs_rows_fwd_h<R, MODE, FK><<<persistent_grid(1, units), K::THREADS, sm, s>>>(p);
+  RowStage st;   // nothing staged: the rows' planes, to be prefetched
+  plan_row_stage(p.cin, p.in, p.ibs, p.nx, p.pre, 1, sm, st, 0);
+  rs_rows_fwd_h<R, MODE, FK><<<persistent_grid(1, units), K::THREADS, sm, s>>>(p, st);
   XL_CHECK_LAUNCH("rs_rows_fwd_h");
   return XL_OK;
 }
