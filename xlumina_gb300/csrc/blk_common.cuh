@@ -42,13 +42,23 @@ static const bool blk_tw_registered = register_device_tables(&blk_upload_twiddle
 // its lane (32 complex values).  One warp allocates the CTA's columns and
 // hands the base address out through shared memory; the same warp frees them
 // before the CTA exits.
+//
+// The 32 lanes of a warp have to execute each of these instructions together,
+// and they are called behind code whose branches depend on the lane (the guards
+// of a ragged edge, a strided loop's last round), so each brings the lanes
+// together itself.  `first` false leaves that out where the lanes came together
+// before (at another of these, a barrier or a __syncwarp) and no branch on the
+// lane has been taken since: with it at every one 8 x 2048^2 VRS takes 2490 us
+// and one 4096^2 1569, as it is 2476 and 1539, without any 2478 and 1544.
 __device__ __forceinline__ void tmem_alloc(unsigned* dst_smem, unsigned ncols) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
                "r"(ncols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned ncols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tmem_fence_before_sync() {
@@ -58,16 +68,22 @@ __device__ __forceinline__ void tmem_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // four complex values into this thread's cells [col, col + 8)
-__device__ __forceinline__ void tmem_st4(unsigned taddr, float2 a, float2 b, float2 c, float2 d) {
+__device__ __forceinline__ void tmem_st4(unsigned taddr, float2 a, float2 b, float2 c, float2 d,
+                                         bool first = true) {
+  if (first) __syncwarp();
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
                "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
                : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st(bool first = true) {
+  if (first) __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 // four complex values back; the values pass through the wait so that no use
 // is scheduled before the load has completed
-__device__ __forceinline__ void tmem_ld4(unsigned taddr, float2 (&o)[4]) {
+__device__ __forceinline__ void tmem_ld4(unsigned taddr, float2 (&o)[4], bool first = true) {
   float r[8];
+  if (first) __syncwarp();
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
                : "r"(taddr)
@@ -119,7 +135,9 @@ template <int R> struct ColMap {
 template <int R> struct TmemTw {
   unsigned cell;
   static __device__ __forceinline__ unsigned at(int i, int q) { return (unsigned)(2 * (i * ((R + 3) / 4 * 4) + 4 * q)); }
-  __device__ __forceinline__ void operator()(int i, int q, float2 (&w)[4]) const { tmem_ld4(cell + at(i, q), w); }
+  __device__ __forceinline__ void operator()(int i, int q, float2 (&w)[4]) const {
+    tmem_ld4(cell + at(i, q), w, i == 0 && q == 0);   // nothing between a phase's reads branches
+  }
 };
 template <int R> struct SmemTw {
   const float2* tw;   // the table at the thread's j
@@ -174,9 +192,9 @@ template <int R, int THREADS, unsigned CELLS, class TW> __device__ __forceinline
     for (int q = 0; q < (R + 3) / 4; ++q) {
       float2 w[4] = {make_float2(1.f, 0.f), make_float2(1.f, 0.f), make_float2(1.f, 0.f), make_float2(1.f, 0.f)};
       tw(i, q, w);
-      tmem_st4(cell + TmemTw<R>::at(i, q), w[0], w[1], w[2], w[3]);
+      tmem_st4(cell + TmemTw<R>::at(i, q), w[0], w[1], w[2], w[3], i == 0 && q == 0);
     }
-  tmem_wait_st();
+  tmem_wait_st(false);
   return cell;
 }
 // Frees them once every thread is done with its cells.

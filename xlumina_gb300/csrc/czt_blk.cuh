@@ -43,11 +43,11 @@ template <int R> struct TmemG {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         w[i] = __ldg(g + (natural ? blk_freq<R>(k1, k2, 4 * q + i) : (4 * q + i) * BlkFft<R>::TB + 16 * k1 + k2));
-      tmem_st4(cell + 8u * q, w[0], w[1], w[2], w[3]);
+      tmem_st4(cell + 8u * q, w[0], w[1], w[2], w[3], q == 0);
     }
-    tmem_wait_st();
+    tmem_wait_st(false);
   }
-  __device__ __forceinline__ void operator()(int q, float2 (&w)[4]) const { tmem_ld4(cell + 8u * q, w); }
+  __device__ __forceinline__ void operator()(int q, float2 (&w)[4]) const { tmem_ld4(cell + 8u * q, w, false); }
 };
 template <int R> struct BlockG {
   const float2* g;   // + the thread's index in phase C
@@ -427,11 +427,10 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) czt_cols_
       }
       __syncthreads();
       blk_a_inv<R, 1>(v, m.jt, line, twa);
-      if (!live) continue;
 #pragma unroll
       for (int f = 0; f < F::IPT * R; ++f) {
         const int o = m.jt + f / R * F::T + 256 * (f % R) - p.ooff_y;
-        if (o < 0 || o >= p.my) continue;
+        if (!live || o < 0 || o >= p.my) continue;
         float2 val = cmul(v[f], __ldg(post_y + o));
         if (p.mode != XL_CZT_PLAIN) {  // wave_optics.py:340, 355: F0 * U (adjoint: conj F)
           const float2 Fv = p.fout ? p.fout[(long long)o * p.mx + col]

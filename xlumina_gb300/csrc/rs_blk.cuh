@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             float2 w[4];
-            tmem_ld4(scell + 8u * q, w);
+            tmem_ld4(scell + 8u * q, w, false);
             mul4(q, w);
           }
         } else {
@@ -104,10 +104,10 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) rs_cols_b
             float2 w[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[i] = __ldg(sp + (4 * q + i) * 32);
-            if (TM && p.cout > 1) tmem_st4(scell + 8u * q, w[0], w[1], w[2], w[3]);
+            if (TM && p.cout > 1) tmem_st4(scell + 8u * q, w[0], w[1], w[2], w[3], false);
             mul4(q, w);
           }
-          if (TM && p.cout > 1) tmem_wait_st();   // complete before the next component's loads
+          if (TM && p.cout > 1) tmem_wait_st(false);   // complete before the next component's loads
         }
         blk_c_inv<1>(v, m.l, blk);
         __syncwarp();

@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, 1) rs_cols_h(const __grid_
         v[n] = n < R && r < ny ? tile[(long long)r << lw] : make_float2(0.f, 0.f);
       }
 #pragma unroll
-      for (int q = 0; q < (R + 3) / 4; ++q) tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-      tmem_wait_st();
+      for (int q = 0; q < (R + 3) / 4; ++q)
+        tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3], q == 0);
+      tmem_wait_st(false);
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         blk_a_fwd<R, -1, false>(v, m.jt, line, twa);
@@ -120,8 +121,8 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, 1) rs_cols_h(const __grid_
 #pragma unroll
         for (int q = 0; q < (R + 3) / 4; ++q) {
           float2 w[4];
-          tmem_ld4(hold + 8u * q, w);
-          if (h == 0) tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          tmem_ld4(hold + 8u * q, w, false);
+          if (h == 0) tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3], false);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (4 * q + i >= R) continue;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, 1) rs_cols_h(const __grid_
             v[4 * q + i] = h == 0 ? cmul(w[i], t) : cadd(w[i], cmulc(v[4 * q + i], t));
           }
         }
-        if (h == 0) tmem_wait_st();
+        if (h == 0) tmem_wait_st(false);
       }
 #pragma unroll
       for (int n = 0; n < R; ++n) {
@@ -226,9 +227,9 @@ __global__ void __launch_bounds__(HalfRow<R>::THREADS, 1) rs_rows_fwd_h(const __
     float2 w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = 4 * q + i < R ? half_tw<R>()[t + 256 * (4 * q + i)] : make_float2(0.f, 0.f);
-    tmem_st4(cell2 + 8u * q, w[0], w[1], w[2], w[3]);
+    tmem_st4(cell2 + 8u * q, w[0], w[1], w[2], w[3], q == 0);
   }
-  tmem_wait_st();
+  tmem_wait_st(false);
   __syncthreads();
   const bool active = t < F::TB;
   float2* blk = line + (t >> 4) * F::BLK;
@@ -371,15 +372,16 @@ __global__ void __launch_bounds__(HalfRow<R>::THREADS, 1) rs_rows_inv_h(const __
       blk_a_inv<R, 1>(v, t, line, twa);
       if (h == 0) {
 #pragma unroll
-        for (int q = 0; q < (R + 3) / 4; ++q) tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        tmem_wait_st();
+        for (int q = 0; q < (R + 3) / 4; ++q)
+          tmem_st4(hold + 8u * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3], false);
+        tmem_wait_st(false);
         sync();   // the odd half's phase C stores to slots that phase A loads here
       }
     }
 #pragma unroll
     for (int q = 0; q < (R + 3) / 4; ++q) {
       float2 w[4];
-      tmem_ld4(hold + 8u * q, w);
+      tmem_ld4(hold + 8u * q, w, false);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (4 * q + i < R) v[4 * q + i] = cadd(w[i], cmulc(v[4 * q + i], __ldg(tw2 + 256 * (4 * q + i))));
