@@ -175,10 +175,15 @@ def keep_for_capture(t):
 
 
 def is_plain_cuda(t) -> bool:
-    """Whether a kernel of the library can read the tensor's memory: an ordinary
-    tensor of the current device (no subclass, no functorch transform's wrapper,
-    no lazily negated view)."""
-    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and
+    """Whether a kernel of the library may take the place of torch operations on
+    the tensor's memory: an ordinary tensor of the current device (no subclass,
+    no functorch transform's wrapper, no lazily negated view), and nobody records
+    or intercepts the operations (a tracer would keep the output's allocation and
+    miss the kernel that fills it)."""
+    if torch.compiler.is_compiling():
+        return False
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and not torch.jit.is_tracing() and
+            not torch._C._len_torch_dispatch_stack() and t.is_cuda and
             t.device.index == torch.cuda.current_device() and not t.is_neg() and
             not torch._C._functorch.is_functorch_wrapped_tensor(t))
 
@@ -260,8 +265,15 @@ def rs_wrapped_offsets(x: np.ndarray, P: int) -> np.ndarray:
 _geometry_cache: "collections.OrderedDict" = collections.OrderedDict()
 
 
+def _geometry(x, y):
+    """(pixel diagonal, largest radius) of a grid."""
+    return np.sqrt((x[1] - x[0]) ** 2 + (y[1] - y[0]) ** 2), np.sqrt((x ** 2).max() + (y ** 2).max())
+
+
 def _grid_geometry(x, y):
-    """(pixel diagonal, largest radius) of a grid, cached by its values."""
+    """The same, cached by the grid's values (a compiler follows the arithmetic only)."""
+    if torch.compiler.is_compiling():
+        return _geometry(x, y)
     x, y = as_grid(x), as_grid(y)
     key = (array_key(x), array_key(y))
     with _LOCK:
@@ -269,7 +281,7 @@ def _grid_geometry(x, y):
         if g is not None:
             _geometry_cache.move_to_end(key)
             return g
-    g = (np.sqrt((x[1] - x[0]) ** 2 + (y[1] - y[0]) ** 2), np.sqrt((x ** 2).max() + (y ** 2).max()))
+    g = _geometry(x, y)
     with _LOCK:
         _geometry_cache[key] = g
         while len(_geometry_cache) > 64:
@@ -283,7 +295,7 @@ def quality_factor(x, y, wavelength, z):
     dr_real, rmax = _grid_geometry(x, y)
     if isinstance(z, torch.Tensor):
         z = z.detach().to(torch.float64)
-        if z.numel() and is_plain_cuda(z):
+        if is_plain_cuda(z) and z.numel():
             z = z.contiguous()
             out = torch.empty_like(z)
             _lib.check(lib().xl_quality_factor(stream_handle(), z.data_ptr(), z.numel(), float(wavelength), float(rmax),
