@@ -59,15 +59,19 @@ struct RsGeom {
   ffloat z2, invl;
   float zf, k, sgn;   // z, 2 pi / lambda, sign of z (the exponent's sign)
 };
-__device__ __forceinline__ RsGeom rs_geom(double z, double inv_lambda, float k) {
+__device__ __forceinline__ RsGeom rs_geom(double z, ffloat inv_lambda, float k) {
   RsGeom g;
   const ffloat zz = ff_split(z);
   g.z2 = ff_mul(zz, zz);
-  g.invl = ff_split(inv_lambda);
+  g.invl = inv_lambda;
   g.zf = (float)z;
   g.k = k;
   g.sgn = z > 0 ? 1.f : -1.f;
   return g;
+}
+
+__device__ __forceinline__ RsGeom rs_geom(double z, double inv_lambda, float k) {
+  return rs_geom(z, ff_split(inv_lambda), k);
 }
 
 // s = X^2 + Y^2 + z^2 in float-float for an offset split into float-float

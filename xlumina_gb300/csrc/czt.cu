@@ -313,6 +313,8 @@ static int czt_run(void* stream, const XlCztArgs* a, int stage) {
   p.x = a->x; p.y = a->y; p.xo = a->xout; p.yo = a->yout;
   p.z = a->z;
   p.inv_lambda = a->wavelength > 0 ? 1.0 / a->wavelength : 0.0;
+  p.invl_hi = (float)p.inv_lambda;
+  p.invl_lo = (float)(p.inv_lambda - (double)p.invl_hi);
   p.k = a->wavelength > 0 ? (float)(2.0 * M_PI / a->wavelength) : 0.f;
   p.cte = make_float2((float)a->cte_re, (float)(a->adjoint ? -a->cte_im : a->cte_im));
   p.pre_x = (const float2*)a->pre_x; p.g_x = (const float2*)a->g_x; p.post_x = (const float2*)a->post_x;

@@ -13,11 +13,11 @@
 // 50 %; without the phases between the two barriers 8 x 2048^2 high-NA tables
 // take 666 of 780 us, without sines and cosines 686), the y transform the
 // shared-memory pipe, as the RS column pass.  Measured, x and y transform (us;
-// Stockham engine before): 4 x 2048^2 -> 1024^2 full focus 646 and 278 (888 and
-// 288), 8 of its Ez alone 751 and 197 (845 and 208), their adjoint 163 and 318
-// (196 and 420); 16 x 1024^2 -> 512^2 behind a lens 222 and 94 (295 and 103),
-// adjoint 95 and 190 (117 and 221); 2 x 1500^2 -> 301^2 VCZT 176 and 32 (216
-// and 31).
+// Stockham engine before): 4 x 2048^2 -> 1024^2 full focus 628 and 278 (888 and
+// 288), 8 of its Ez alone 740 and 197 (845 and 208), their adjoint 158 and 318
+// (196 and 420); 16 x 1024^2 -> 512^2 behind a lens 217 and 94 (295 and 103),
+// adjoint 85 and 190 (117 and 221), with a distance for each entry 320 and 171
+// (438 and 140); 2 x 1500^2 -> 301^2 VCZT 172 and 32 (216 and 31).
 #pragma once
 
 #include <math.h>
@@ -191,6 +191,8 @@ __global__ void __launch_bounds__(CztRowB<R, NC, FK>::THREADS, CztRowB<R, NC, FK
     const bool live = r < ny;
     const int c = cg;
     const bool act = live && c < p.cout;
+    RsGeom geo;          // where no plane of F is at hand: its constants, with Y^2 of
+    int geo_row = -1;    // this row added to z^2 (float64 splits, once a row)
     // the fused program, the VCZT Ez and the input-plane transfer function on
     // NPX pixels: (row of the group, column) of pixel q from at(q), results to
     // put(q, e)
@@ -229,7 +231,21 @@ __global__ void __launch_bounds__(CztRowB<R, NC, FK>::THREADS, CztRowB<R, NC, FK
             }
           }
           // wave_optics.py:341 (F on the input plane); the adjoint applies conj(F0) here
-          float2 Fv = st.aux >= 0 ? ((const float2*)(stage + st.aux))[(rr - r0) * nx + n] : p.fin ? p.fin[px[q].pix] : rs_kernel_value(p.x[n], p.y[rr], zd, p.inv_lambda, p.k);
+          float2 Fv;
+          if (st.aux >= 0) {
+            Fv = ((const float2*)(stage + st.aux))[(rr - r0) * nx + n];
+          } else if (p.fin) {
+            Fv = p.fin[px[q].pix];
+          } else {
+            if (rr != geo_row) {
+              geo_row = rr;
+              geo = rs_geom(zd, ffloat{p.invl_hi, p.invl_lo}, p.k);
+              const ffloat Y = ff_split(p.y[rr]);
+              geo.z2 = ff_add(geo.z2, ff_mul(Y, Y));
+            }
+            const ffloat X = ff_split(p.x[n]);
+            Fv = rs_value_s(geo, ff_add(geo.z2, ff_mul(X, X)));
+          }
           if (p.adjoint) Fv = cconj(Fv);
 #pragma unroll
           for (int i = 0; i < 3; ++i) e[q][i] = cmul(e[q][i], Fv);
@@ -244,35 +260,32 @@ __global__ void __launch_bounds__(CztRowB<R, NC, FK>::THREADS, CztRowB<R, NC, FK
       // line (no barrier).  Few, since the fused program's code is laid out once
       // for each and the instruction cache is what bounds it (8 x 2048^2 high-NA
       // tables: 8 at a time 910 us, 4 780, 2 762, 1 796; unrolled over all, with
-      // the results in registers, 1181; 16 x 1024^2 behind a lens: 4 253, 2 221).  Positions outside the window take a valid pixel and
-      // are zeroed below; a step all outside is skipped.
+      // the results in registers, 1181; 16 x 1024^2 behind a lens: 4 253, 2 221).
+      // Its j-th element is at t + T j: those inside the window, j0 to j1, follow
+      // each other; one past the end takes a valid pixel.
       const int g2 = min(gi, ny - 1 - r0);
       constexpr int N = F::IPT * R, NP = 2;
       float2* own = line + blk_slot(t);
-      auto pos = [&](int f) { return t + f / R * F::T + 256 * (f % R) - p.ioff_x; };
-      auto slot = [&](int f) { return f % R * F::BLK + f / R * (F::T / 16) * 18; };
+      const int at0 = t - p.ioff_x;   // position in the window of element 0
+      const int j0 = at0 < 0 ? (F::T - 1 - at0) / F::T : 0;
+      const int j1 = at0 < nx ? min((nx - 1 - at0) / F::T + 1, N) : 0;
 #pragma unroll 1
-      for (int f0 = 0; f0 < N; f0 += NP) {
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          const int n = pos(f0 + q);
-          any = any || (f0 + q < N && n >= 0 && n < nx);
-        }
-        if (!any) continue;
+      for (int j = j0; j < j1; j += NP) {
         pixels(std::integral_constant<int, NP>{},
                [&](int q, int& g, int& n) {
                  g = g2;
-                 n = min(max(pos(f0 + q), 0), nx - 1);
+                 n = min(at0 + (j + q) * F::T, nx - 1);
                },
                [&](int q, const float2 (&e)[3]) {
-                 if (f0 + q < N) own[slot(f0 + q)] = e[0];
+                 const int f = j + q;
+                 if (f < j1) own[f / F::IPT * F::BLK + f % F::IPT * (F::T / 16) * 18] = e[0];
                });
       }
 #pragma unroll
       for (int f = 0; f < N; ++f) {
-        const int n = pos(f);
-        v[f] = (act && n >= 0 && n < nx) ? cmul(own[slot(f)], __ldg(pre_x + n)) : make_float2(0.f, 0.f);
+        const int n = at0 + f / R * F::T + 256 * (f % R);
+        v[f] = (act && n >= 0 && n < nx) ? cmul(own[f % R * F::BLK + f / R * (F::T / 16) * 18], __ldg(pre_x + n))
+                                         : make_float2(0.f, 0.f);
       }
     } else {
       const int lim = min(K::G, ny - r0) * nx;

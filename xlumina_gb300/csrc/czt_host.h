@@ -23,6 +23,7 @@ struct CztLaunch {
   const double* xo;
   const double* yo;
   double z, inv_lambda;
+  float invl_hi, invl_lo;                 // inv_lambda as float-float
   float k;
   float2 cte;
   const float2* pre_x;   // nx
