@@ -13,11 +13,11 @@
 // 50 %; without the phases between the two barriers 8 x 2048^2 high-NA tables
 // take 666 of 780 us, without sines and cosines 686), the y transform the
 // shared-memory pipe, as the RS column pass.  Measured, x and y transform (us;
-// Stockham engine before): 4 x 2048^2 -> 1024^2 full focus 628 and 278 (888 and
-// 288), 8 of its Ez alone 740 and 197 (845 and 208), their adjoint 158 and 318
-// (196 and 420); 16 x 1024^2 -> 512^2 behind a lens 217 and 94 (295 and 103),
-// adjoint 85 and 190 (117 and 221), with a distance for each entry 320 and 171
-// (438 and 140); 2 x 1500^2 -> 301^2 VCZT 172 and 32 (216 and 31).
+// Stockham engine before): 4 x 2048^2 -> 1024^2 full focus 628 and 263 (888 and
+// 288), 8 of its Ez alone 740 and 184 (845 and 208), their adjoint 158 and 283
+// (196 and 420); 16 x 1024^2 -> 512^2 behind a lens 217 and 88 (295 and 103),
+// adjoint 85 and 176 (117 and 221), with a distance for each entry 320 and 133
+// (438 and 140); 2 x 1500^2 -> 301^2 VCZT 172 and 29 (216 and 31).
 #pragma once
 
 #include <math.h>
@@ -37,14 +37,12 @@ namespace xl {
 template <int R> struct TmemG {
   unsigned cell;
   __device__ __forceinline__ void fill(const float2* g, bool natural, int k1, int k2) const {
+    float2 w[16];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float2 w[4];
+    for (int i = 0; i < 16; ++i)
+      w[i] = __ldg(g + (natural ? blk_freq<R>(k1, k2, i) : i * BlkFft<R>::TB + 16 * k1 + k2));
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        w[i] = __ldg(g + (natural ? blk_freq<R>(k1, k2, 4 * q + i) : (4 * q + i) * BlkFft<R>::TB + 16 * k1 + k2));
-      tmem_st4(cell + 8u * q, w[0], w[1], w[2], w[3], q == 0);
-    }
+    for (int q = 0; q < 4; ++q) tmem_st4(cell + 8u * q, w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3], q == 0);
     tmem_wait_st(false);
   }
   __device__ __forceinline__ void operator()(int q, float2 (&w)[4]) const { tmem_ld4(cell + 8u * q, w, false); }
@@ -350,8 +348,12 @@ __global__ void __launch_bounds__(CztRowB<R, NC, FK>::THREADS, CztRowB<R, NC, FK
 // y transform over groups of CW columns, with the epilogue.  Persistent: CTAs
 // walk the (column group, batch entry) units, groups fastest, a unit's
 // components one after the other; cu > 1: a unit for each component, where
-// there are few of them.
-template <int R>
+// there are few of them.  VALUE: the transfer function F0 is evaluated at each
+// output sample (a distance of its own for every entry, or a first call, which
+// has no plane of it yet); its code and registers stay out of the other kernel
+// (16 x 1024^2 -> 512^2 adjoint: 176 us, one kernel for both 194; with a distance
+// for each entry 133).
+template <int R, bool VALUE>
 __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) czt_cols_b(const __grid_constant__ CztLaunch p, int cu) {
   using F = BlkFft<R>;
   using K = RsColB<R>;
@@ -389,9 +391,16 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) czt_cols_
   const bool fold = p.adjoint && p.mode == XL_CZT_VECTOR;
   const int ny = p.ny, lw = p.lw;
   const int groups = (p.mx + K::CW - 1) / K::CW;
+  const int units = groups * cu * p.B;
+  // with chirps of its own for every entry a CTA takes a run of units, so that
+  // the spectrum it holds changes once or twice
+  const bool runs = VALUE && p.zb;
+  const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int first = runs ? (int)blockIdx.x * per : (int)blockIdx.x;
+  const int last = runs ? min(first + per, units) : units, step = runs ? 1 : (int)gridDim.x;
   int held = 0;
 #pragma unroll 1
-  for (int u = blockIdx.x; u < groups * cu * p.B; u += gridDim.x) {
+  for (int u = first; u < last; u += step) {
     const int g = u % groups, b = u / groups / cu;
     const int c0 = cu > 1 ? u / groups % cu : 0, c1 = cu > 1 ? c0 + 1 : p.cout;
     const int col = g * K::CW + m.wc;
@@ -440,14 +449,26 @@ __global__ void __launch_bounds__(RsColB<R>::THREADS, RsColB<R>::MINB) czt_cols_
       }
       __syncthreads();
       blk_a_inv<R, 1>(v, m.jt, line, twa);
+      RsGeom geo;
+      ffloat XX;
+      if constexpr (VALUE) {
+        geo = rs_geom(zd, ffloat{p.invl_hi, p.invl_lo}, p.k);
+        const ffloat X = ff_split(p.xo[live ? col : 0]);
+        XX = ff_mul(X, X);
+      }
 #pragma unroll
       for (int f = 0; f < F::IPT * R; ++f) {
         const int o = m.jt + f / R * F::T + 256 * (f % R) - p.ooff_y;
         if (!live || o < 0 || o >= p.my) continue;
         float2 val = cmul(v[f], __ldg(post_y + o));
-        if (p.mode != XL_CZT_PLAIN) {  // wave_optics.py:340, 355: F0 * U (adjoint: conj F)
-          const float2 Fv = p.fout ? p.fout[(long long)o * p.mx + col]
-                                   : rs_kernel_value(p.xo[col], p.yo[o], zd, p.inv_lambda, p.k);
+        if (VALUE || p.mode != XL_CZT_PLAIN) {  // wave_optics.py:340, 355: F0 * U (adjoint: conj F)
+          float2 Fv;
+          if constexpr (VALUE) {
+            const ffloat Y = ff_split(p.yo[o]);
+            Fv = rs_value_s(geo, ff_add(ff_add(geo.z2, ff_mul(Y, Y)), XX));
+          } else {
+            Fv = p.fout[(long long)o * p.mx + col];
+          }
           val = p.adjoint ? cmulc(val, Fv) : cmul(val, Fv);
         }
         val = cmul(val, cte);
@@ -509,11 +530,11 @@ template <int R> int czt_blk_rows(cudaStream_t s, const CztLaunch& p) {
   return launch_czt_rows_b<R, 1>(s, p);
 }
 
-template <int R> int czt_blk_cols(cudaStream_t s, const CztLaunch& p) {
+template <int R, bool VALUE> static int launch_czt_cols_b(cudaStream_t s, const CztLaunch& p) {
   using K = RsColB<R>;
   const size_t sm = K::SMEM + (!K::TM && p.nat_y ? (size_t)BlkFft<R>::P * 8 : 0);
   int per_sm;
-  if (int rc = launch_ready<czt_cols_b<R>>(K::THREADS, sm, &per_sm, "czt_cols_b")) return rc;
+  if (int rc = launch_ready<czt_cols_b<R, VALUE>>(K::THREADS, sm, &per_sm, "czt_cols_b")) return rc;
   // a unit for each component where there are fewer than two rounds of units
   // (2 x 301^2 VCZT outputs, 76 units for 152 SMs: 32 us, 41 without; 4 x
   // 1024^2, 512 units: 291 and 278), unless the VCZT adjoint folds one into the
@@ -521,9 +542,13 @@ template <int R> int czt_blk_cols(cudaStream_t s, const CztLaunch& p) {
   const long long units = (long long)p.B * ((p.mx + K::CW - 1) / K::CW);
   const bool fold = p.adjoint && p.mode == XL_CZT_VECTOR;
   const int cu = !fold && units < 2LL * per_sm * device_sms() ? p.cout : 1;
-  czt_cols_b<R><<<persistent_grid(per_sm, units * cu), K::THREADS, sm, s>>>(p, cu);
+  czt_cols_b<R, VALUE><<<persistent_grid(per_sm, units * cu), K::THREADS, sm, s>>>(p, cu);
   XL_CHECK_LAUNCH("czt_cols_b");
   return XL_OK;
+}
+
+template <int R> int czt_blk_cols(cudaStream_t s, const CztLaunch& p) {
+  return p.mode != XL_CZT_PLAIN && !p.fout ? launch_czt_cols_b<R, true>(s, p) : launch_czt_cols_b<R, false>(s, p);
 }
 
 }  // namespace xl
