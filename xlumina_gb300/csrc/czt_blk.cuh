@@ -63,11 +63,13 @@ template <int R> __device__ __forceinline__ void smem_g_fill(float2* dst, const 
 }
 
 // Thread organisation of the x transform: RowB's, with the CTAs per SM that
-// the registers are sized for.  One component: three of 256 threads, two (128
-// registers) for a fused program of several ops, whose pixels' trig is in
-// flight together.
+// the registers are sized for.  One component: three of 256 threads, but from
+// 3072 points two (128 registers, and twice the room for staged planes) for a
+// fixed program of several ops (the high-NA table's, 8 fields: 2048^2 -> 1024^2
+// 738 us, with three CTAs 803; 1800^2 -> 1000^2 641, 635; 4 x 1600^2 -> 900^2, a
+// step shorter, 276 with two, 224 with three).
 template <int R, int NC, class FK = FixedKinds<>> struct CztRowB : RowB<R, NC> {
-  static constexpr int MB = NC == 1 ? (FK::n > 1 ? 2 : 3) : 1;
+  static constexpr int MB = NC == 1 ? (FK::n > 1 && R >= 12 ? 2 : 3) : 1;
 };
 
 // Bytes of the x transform's shared memory before its stage.
@@ -507,26 +509,25 @@ template <int R, int NC, class FK = FixedKinds<>> static int launch_czt_rows_b(c
 }
 
 template <int R> int czt_blk_rows(cudaStream_t s, const CztLaunch& p) {
-  // the forward programs of the tables and of the full focus get a kernel with
-  // their op kinds fixed, at the lengths they have: the high-NA table's LCD,
-  // sSLM and lens Ez row, an sSLM before the lens (4 x 2048^2 -> 1024^2: 646 us,
-  // with the generic program 712), the 4f table's thin lens and its second
-  // phase SLM
+  // programs that get a kernel with their op kinds fixed, at every length: an
+  // sSLM before the high-NA lens; an LCD, an sSLM and the lens's Ez row; a thin
+  // lens; a phase SLM.  Fixed against generic, rows in us at 1024, 1536, 2048,
+  // 2560, .. points: sSLM and lens, 33 x 600^2 440 and 488, 14 x 900^2 490 and
+  // 528, 7 x 1300^2 439 and 480, 4 x 1600^2 455 and 498 (4 x 2048^2 646 and 712);
+  // the Ez row 320 and 380, 307 and 368, 330 and 392, 224 and 270; a thin lens
+  // 170 and 185 at 1024 points, 134 and 153 for 2 x 2040^2 at 4096; a phase SLM
+  // 150 and 169 at 1536, 132 and 153 at 4096.
   if (p.cout > 1) {
     using HighNa = FixedKinds<XL_OP_SSLM, XL_OP_HIGHNA>;
-    if constexpr (R >= 12)
-      if (HighNa::matches(p.pre)) return launch_czt_rows_b<R, 3, HighNa>(s, p);
+    if (HighNa::matches(p.pre)) return launch_czt_rows_b<R, 3, HighNa>(s, p);
     return launch_czt_rows_b<R, 3>(s, p);
   }
   using HighNaEz = FixedKinds<XL_OP_LCD, XL_OP_SSLM, XL_OP_HIGHNA_EZ>;
   using LensOnly = FixedKinds<XL_OP_SEPMASK>;
   using SlmOnly = FixedKinds<XL_OP_PHASE>;
-  if constexpr (R >= 12)
-    if (HighNaEz::matches(p.pre)) return launch_czt_rows_b<R, 1, HighNaEz>(s, p);
-  if constexpr (R == 6 || R == 8)
-    if (LensOnly::matches(p.pre)) return launch_czt_rows_b<R, 1, LensOnly>(s, p);
-  if constexpr (R == 4)
-    if (SlmOnly::matches(p.pre)) return launch_czt_rows_b<R, 1, SlmOnly>(s, p);
+  if (HighNaEz::matches(p.pre)) return launch_czt_rows_b<R, 1, HighNaEz>(s, p);
+  if (LensOnly::matches(p.pre)) return launch_czt_rows_b<R, 1, LensOnly>(s, p);
+  if (SlmOnly::matches(p.pre)) return launch_czt_rows_b<R, 1, SlmOnly>(s, p);
   return launch_czt_rows_b<R, 1>(s, p);
 }
 
