@@ -49,3 +49,19 @@ def test_chirp_z(nx, mx):
     for op in (engine.op_phase(P[0]), engine.op_lens(x, y, 0.633, (0.8 * nx, 0.9 * nx), (60.0 * nx, 70.0 * nx), False)):
         call = lambda c, pre: engine.czt_propagate(c, x, y, 0.633, 60.0 * nx, xo, yo, "scalar", pre=pre)  # noqa: E731
         _same(call(e[:1], [op]), call(engine.apply_ops(e[:1], [op], ny, nx), []))
+
+
+# x transforms of 1024, 1536, .. 4096 points, then of 5120 and 8192
+@pytest.mark.parametrize("nx", [300, 513, 1000, 1025, 1500, 1793, 2047, 2051, 3590])
+def test_rs(nx):
+    from xlumina_gb300 import engine
+    ny = 41
+    x, y = np.linspace(-1.0, 1.0, nx) * nx, np.linspace(-1.0, 1.0, ny) * ny
+    e = _rand(2, ny, nx)
+    e = [e[0], e[1]]
+    P = [_plane(k, 2, ny, nx) for k in range(2)]
+    call = lambda c, pre: engine.rs_propagate(c, x, y, 0.633, 5.0e4, len(c) == 2, pre=pre)  # noqa: E731
+    slm = [engine.op_phase(P[0])]
+    _same(call(e[:1], slm), call(engine.apply_ops(e[:1], slm, ny, nx), []))
+    for ops in ([engine.op_sslm(P[0], P[1])], [engine.op_lcd(P[0], P[1]), engine.op_lp(0.3)]):
+        _same(call(e, ops), call(engine.apply_ops(e, ops, ny, nx), []))

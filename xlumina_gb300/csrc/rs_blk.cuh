@@ -687,27 +687,16 @@ template <int R, int COUT, bool EPI, bool POL = false> static int launch_rows_in
 
 template <int R> int rs_blk_rows(cudaStream_t st, const RsLaunch& p, bool inverse) {
   if (!inverse) {
-    // the programs of the benchmarks' fields get a kernel with their op kinds
-    // fixed: a phase SLM before scalar RS, a double-phase SLM before VRS (the
-    // building block), an LCD before a polarizer and VRS
+    // programs that get a kernel with their op kinds fixed: a phase SLM before
+    // scalar RS, a double-phase SLM before VRS, an LCD before a polarizer and VRS
+    // (us, generic and fixed, at 1024 and 1536 points: 75 x 400^2 107 and 98, 288
+    // and 271, 233 and 212; 20 x 768^2 111 and 103, 256 and 245, 205 and 185)
     using SlmOnly = FixedKinds<XL_OP_PHASE>;
     using LcdOnly = FixedKinds<XL_OP_LCD>;
-    if (p.pol) {
-      if constexpr (R >= 8)
-        if (LcdOnly::matches(p.pre)) return launch_rows_fwd_b<R, 4, LcdOnly>(st, p);
-      return launch_rows_fwd_b<R, 4>(st, p);
-    }
-    if (p.cout == 1) {
-      if constexpr (R >= 8)
-        if (SlmOnly::matches(p.pre)) return launch_rows_fwd_b<R, 1, SlmOnly>(st, p);
-      return launch_rows_fwd_b<R, 1>(st, p);
-    }
     using SlmsOnly = FixedKinds<XL_OP_SSLM>;
-    if (p.cin == 2) {
-      if constexpr (R >= 8)
-        if (SlmsOnly::matches(p.pre)) return launch_rows_fwd_b<R, 2, SlmsOnly>(st, p);
-      return launch_rows_fwd_b<R, 2>(st, p);
-    }
+    if (p.pol) return LcdOnly::matches(p.pre) ? launch_rows_fwd_b<R, 4, LcdOnly>(st, p) : launch_rows_fwd_b<R, 4>(st, p);
+    if (p.cout == 1) return SlmOnly::matches(p.pre) ? launch_rows_fwd_b<R, 1, SlmOnly>(st, p) : launch_rows_fwd_b<R, 1>(st, p);
+    if (p.cin == 2) return SlmsOnly::matches(p.pre) ? launch_rows_fwd_b<R, 2, SlmsOnly>(st, p) : launch_rows_fwd_b<R, 2>(st, p);
     return launch_rows_fwd_b<R, 3>(st, p);
   }
   if (p.pol) {

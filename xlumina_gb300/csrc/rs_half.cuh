@@ -516,10 +516,16 @@ template <int R, int COUT, bool EPI> static int launch_rows_inv_h(cudaStream_t s
 
 template <int R> int rs_half_rows(cudaStream_t st, const RsLaunch& p, bool inverse) {
   if (!inverse) {
+    // the fixed programs of rs_blk_rows (us, generic and fixed: LCD and polarizer,
+    // 2 x 2300^2 349 and 346, one 3200^2 334 and 320; SLM 319 and 300, 304 and 277)
     using SlmOnly = FixedKinds<XL_OP_PHASE>;
+    using LcdLp = FixedKinds<XL_OP_LCD, XL_OP_LP>;
+    using SlmsOnly = FixedKinds<XL_OP_SSLM>;
     if (p.cout == 1)
       return SlmOnly::matches(p.pre) ? launch_rows_fwd_h<R, 1, SlmOnly>(st, p) : launch_rows_fwd_h<R, 1>(st, p);
-    return p.cin == 2 ? launch_rows_fwd_h<R, 2>(st, p) : launch_rows_fwd_h<R, 3>(st, p);
+    if (p.cin == 3) return launch_rows_fwd_h<R, 3>(st, p);
+    if (LcdLp::matches(p.pre)) return launch_rows_fwd_h<R, 2, LcdLp>(st, p);
+    return SlmsOnly::matches(p.pre) ? launch_rows_fwd_h<R, 2, SlmsOnly>(st, p) : launch_rows_fwd_h<R, 2>(st, p);
   }
   const bool epi = p.post.nops > 0 || (p.adjoint && p.cout == 3);
   if (p.cout == 1) return epi ? launch_rows_inv_h<R, 1, true>(st, p) : launch_rows_inv_h<R, 1, false>(st, p);
