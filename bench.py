@@ -331,7 +331,7 @@ def run_gpu(args):
         for s in range(3):
             call.stage(s)
     torch.cuda.synchronize()
-    # the column pass's kernel variant, chosen by measurement on this launch
+    # the column pass's kernel variant (one kernel per transform length: the tuner times that)
     from xlumina_gb300 import _lib
     from xlumina_gb300.autotune import VariantTuner, cuda_event_timer
     col_logp = engine.rs_logq(N, N) + 1

@@ -145,7 +145,12 @@ class VariantTuner:
         self._select = select
 
     def _lib_count(self, pass_id, log2_len):
-        from . import engine
+        from . import _lib, engine
+        # lengths of the block engine have one kernel, which every number that the
+        # library accepts selects: there is nothing to choose by measuring
+        czt = (_lib.XL_PASS_CZT_ROWS, _lib.XL_PASS_CZT_COLS)
+        if int(pass_id) == _lib.XL_PASS_RS_COLS or (int(pass_id) in czt and 10 <= int(log2_len) <= 12):
+            return min(1, int(engine.lib().xl_kernel_variant_count(int(pass_id), int(log2_len))))
         return int(engine.lib().xl_kernel_variant_count(int(pass_id), int(log2_len)))
 
     def _lib_select(self, pass_id, log2_len, v):
