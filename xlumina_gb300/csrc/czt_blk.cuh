@@ -9,10 +9,11 @@
 // 256 R that holds the window (2048 onto 1024 samples: 3072 points where a
 // power of two would be 4096).
 //
-// What bounds them: the x transform its fused prologue (the issue rate is 45 to
-// 50 %; without the phases between the two barriers 8 x 2048^2 high-NA tables
-// take 666 of 780 us, without sines and cosines 686), the y transform the
-// shared-memory pipe, as the RS column pass.  Measured, x and y transform (us;
+// What bounds them: the x transform its fused prologue (the issue rate is 47 to
+// 51 %; without the phases between the two barriers 8 x 2048^2 high-NA tables
+// took 666 of 780 us, without sines and cosines 686), the y transform the latency
+// of a column's loads in a CTA that has its SM to itself (issue rate 48 to 50 %,
+// shared-memory pipe 33 to 39 %, DRAM 10 %).  Measured, x and y transform (us;
 // Stockham engine before): 4 x 2048^2 -> 1024^2 full focus 628 and 263 (888 and
 // 288), 8 of its Ez alone 740 and 184 (845 and 208), their adjoint 158 and 283
 // (196 and 420); 16 x 1024^2 -> 512^2 behind a lens 217 and 88 (295 and 103),

@@ -27,10 +27,10 @@ struct CztLaunch {
   float k;
   float2 cte;
   const float2* pre_x;   // nx
-  const float2* g_x;     // Lx, natural order
+  const float2* g_x;     // Lx, in natural or block order (nat_x)
   const float2* post_x;  // mx (includes 1/Lx)
   const float2* pre_y;   // ny
-  const float2* g_y;     // Ly, natural order
+  const float2* g_y;     // Ly, in natural or block order (nat_y)
   const float2* post_y;  // my (includes 1/Ly)
   float2* work;          // B x cout x ny x mxp, column tiles of 2^lw
   XlProg pre;
@@ -58,8 +58,8 @@ inline int czt_tile_w(int logl) {
 }
 
 // The x transform (rows, prologue) and the y transform (columns, epilogue)
-// for Bluestein length 2^LOGL (explicitly instantiated for LOGL = 5..13 in the
-// kernel translation units).
+// for Bluestein length 2^LOGL (explicitly instantiated for LOGL = 5..9 and 13 in
+// the kernel translation units).
 template <int LOGL>
 int czt_rows_launch(cudaStream_t st, const CztLaunch& p);
 template <int LOGL>

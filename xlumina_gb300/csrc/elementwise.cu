@@ -54,8 +54,9 @@ __global__ void mask_kernel(const ElemLaunch p) {
 // exp(i phase) of n phases, two at a time where both arrays are aligned for it
 // (8 and 16 bytes): a warp's accesses are then whole lines, and a thread has
 // four loads in flight.  The kernel writes 8 bytes a phase and reads 4.
-// 16 x 1024^2 take 28 us, 30 at the copy rate (torch.polar on a plane of ones:
-// 53; four phases a thread, whose two 16-byte stores are half lines each: 36).
+// 16 x 1024^2 take 34 us, 30 at the copy rate (torch.polar on a plane of ones:
+// 61).  One launch under the profiler, the last stores still in L2: 28, with
+// four phases a thread, whose two 16-byte stores are half lines each, 36.
 constexpr int MASK_THREADS = 256, MASK_IPT = 4;
 __global__ void __launch_bounds__(MASK_THREADS) phase_mask_kernel(const float* __restrict__ ph,
                                                                   float2* __restrict__ out, long long n, int vec) {
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
         // every load of the pixel before the first sine: their slow paths are
         // branches, past which no load is moved up, and each op's loads were
         // waited for by themselves (8 x 2048^2 LCD, sSLM, lens Ez row: 589 us,
-        // now 485; LCD and polarizer 448 and 352)
+        // now 480; LCD and polarizer 448 and 353)
         g[0] = p.gout[0][go];
         if (p.C > 1 && p.gout[1]) g[1] = p.gout[1][go];
         if (p.C > 2 && p.gout[2]) g[2] = p.gout[2][go];
@@ -282,9 +283,9 @@ __global__ void __launch_bounds__(128) ops_backward_kernel(const OpsBwdLaunch p,
 // Scalar programs of one op, two pixels a thread in 16-byte accesses: a phase
 // SLM with its gradient in a plane per batch entry, and a separable mask (no
 // parameter gradient; the forward's input is not read).  The kernel above, one
-// pixel a thread, does not keep enough bytes in flight: 16 x 1024^2, phase 107
-// us, mask 95; these take 64 and 48 (24 bytes a pixel and 16 at the copy rate: 59
-// and 40).
+// pixel a thread, does not keep enough bytes in flight: 16 x 1024^2, phase 110
+// us, with the input's gradient 121, mask 98; these take 62, 85 and 47 (at the
+// copy rate 59, 79 and 40).
 template <bool IN>
 __global__ void __launch_bounds__(256) phase_backward_kernel(const OpsBwdLaunch p) {
   const long long n2 = (long long)p.ny * p.nx / 2;
@@ -430,8 +431,8 @@ __global__ void __launch_bounds__(MSE_THREADS) plane_sum_partial(const float2* _
 
 // The intensity MSE of three components in tensors of their own (grid z), and
 // its gradient: one launch each instead of three.  A vector light's loss is a
-// chain of short kernels: 1024^2, with the launches around it, 1207 -> 893 us a
-// building block with gradients.
+// chain of short kernels: 1024^2 with gradients, through autograd, 310 us (three
+// runs 308 to 319), with a launch a component 510 (499 to 520).
 struct Vmse {
   const float2* a[3];
   const float2* b[3];

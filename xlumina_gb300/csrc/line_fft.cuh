@@ -72,9 +72,10 @@ struct RowStage {
   int aux;                     // stage offset of a caller's plane of complex values, -1: global memory
   int prm[XL_MAX_OPS][4];      // stage offset of parameter plane i of op k, -1: global memory
   // planes the prologue reads from global memory (not staged, or the lens
-  // coefficient planes); the chirp-z x transform prefetches them into L2 one
-  // row group ahead (in the RS forward row pass, whose planes are all staged
-  // in the benchmarked cases, the prefetch code cost 1.5 % and is left out)
+  // coefficient planes); the chirp-z x transform and the RS rows above 2048
+  // pixels, which stage nothing, prefetch them into L2 one row group ahead (the
+  // shorter RS rows leave it out: where all their planes are staged the code cost
+  // 1.5 %)
   int npf;
   RowStream pf[XL_ROW_PREFETCH];   // soff unused
 };

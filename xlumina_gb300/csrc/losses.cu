@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(LOSS_THREADS) loss_grad(LossIn in, const float
   const int plane = blockIdx.y;
   // one thread of the block forms the plane's constants: in float64 with
   // divisions, which every thread used to do for the one or two pixels it had
-  // (16 x 512^2: 126 us, now 26)
+  // (16 x 512^2: 124 us, now 17; 12 at the copy rate)
   __shared__ float con[4];   // 1 / (S + eps), threshold, and dL/dI_j = con[2] * (u_j-term) + con[3]
   if (threadIdx.x == 0) {
     const double* st = stats + (long long)plane * LOSS_STATS;

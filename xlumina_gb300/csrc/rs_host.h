@@ -30,9 +30,9 @@ struct RsLaunch {
   int lw;                       // log2 of the intermediate's column-tile width (block engine)
 };
 
-// Q = 2^logq is the half transform length: the smallest power of two >= the field side.
-// Q = 2^logq >= the field side, at least 32: the transfer-spectrum row pass
-// takes G = 256 / T rows per CTA, which for Q = 16 (P = 32) exceeds P.
+// Q = 2^logq is the half transform length: the smallest power of two >= the field
+// side, at least 32 (the transfer-spectrum row pass takes G = 256 / T rows per CTA,
+// which for Q = 16, P = 32, exceeds P).
 inline int rs_logq(int ny, int nx) {
   const int n = ny > nx ? ny : nx;
   const int l = ilog2_ceil(n);

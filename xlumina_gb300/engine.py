@@ -653,7 +653,8 @@ def device_offsets(a: np.ndarray, P: int) -> torch.Tensor:
 
 def build_rs_spectra_device(x, y, zd: torch.Tensor, wavelength, dz=False) -> torch.Tensor:
     """Transfer spectra (or dH/dz spectra) for the distances of a device array,
-    one per entry, stacked: shape (len(zd), P*P).  No host synchronisation."""
+    one per entry, stacked: shape (len(zd), points of one spectrum).  No host
+    synchronisation."""
     L = lib()
     ny, nx = len(y), len(x)
     P = 2 << rs_logq(ny, nx)
