@@ -92,7 +92,10 @@ def batch_planes(comps, ny, nx):
     if B > 1 and all(c.dim() == 3 and c.stride(0) == 0 and c.dtype == torch.complex64 and c.is_cuda and
                      c[0].is_contiguous() for c in comps):
         return [c[0] for c in comps], B, 0
-    return [as_field(c).contiguous() for c in comps], B, ny * nx
+    planes = [as_field(c).contiguous() for c in comps]
+    if any(p.numel() < B * ny * nx for p in planes):
+        raise ValueError(f"components of shapes {[tuple(p.shape) for p in planes]} in a batch of {B} fields")
+    return planes, B, ny * nx
 
 
 def as_real_param(a, dev=None):
@@ -313,7 +316,7 @@ def quality_factor(x, y, wavelength, z):
 class JonesOp:
     """One per-pixel operation of a fused program (see XL_OP_* in xlgb.h)."""
 
-    __slots__ = ("kind", "params", "ptrs", "sval", "dval", "keep", "planes")
+    __slots__ = ("kind", "params", "ptrs", "sval", "dval", "keep", "planes", "copies")
 
     def __init__(self, kind, params=(), ptrs=(), sval=(), dval=(), keep=()):
         self.kind = kind
@@ -323,6 +326,7 @@ class JonesOp:
         self.dval = list(dval)
         self.keep = list(keep)
         self.planes = {}             # slot -> plane a one-element tensor parameter was expanded to
+        self.copies = {}             # slot -> the last launch's copies of a plane shared by the batch
 
     @staticmethod
     def is_scalar_tensor(p) -> bool:
@@ -336,10 +340,23 @@ class JonesOp:
     def plane_shape(p, ny, nx):
         return (ny, nx) if p.numel() == 1 else (p.numel(), ny, nx)
 
-    def fill(self, op: _lib.XlOp, ny: int, nx: int) -> None:
+    def plane_batch(self) -> int:
+        """Planes per parameter: the batch of those that have one for every entry,
+        1 if all are shared by it.  An op has one stride for all of them, so a
+        shared plane beside them is copied for every entry."""
+        sizes = {p.numel() if p.dim() < 2 else p.shape[0] for p in self.params
+                 if isinstance(p, torch.Tensor) and (p.dim() == 3 or p.dim() < 2)} - {1}
+        if len(sizes) > 1:
+            raise ValueError(f"mask parameters of one device have batches of {sorted(sizes)} planes")
+        return sizes.pop() if sizes else 1
+
+    def fill(self, op: _lib.XlOp, ny: int, nx: int, batch: int = 1) -> None:
         op.kind = self.kind
         pmask = 0
         pbstride = 0
+        nb = self.plane_batch()
+        if 1 < nb < batch:
+            raise ValueError(f"mask parameters for {nb} entries, a batch of {batch} fields")
         for i, p in enumerate(self.params):
             if self.is_scalar_tensor(p):
                 shape = self.plane_shape(p, ny, nx)
@@ -350,8 +367,11 @@ class JonesOp:
                     self.planes[i] = plane
                 p = keep_for_capture(plane)
             if isinstance(p, torch.Tensor):
-                if p.shape[-2:] != (ny, nx):
+                if p.shape[-2:] != (ny, nx) or not p.numel():
                     raise ValueError(f"mask parameter has shape {tuple(p.shape)}, field is {(ny, nx)}")
+                if nb > 1 and p.numel() == ny * nx:
+                    p = self.copies[i] = p.detach().reshape(1, ny, nx).expand(nb, ny, nx).contiguous()
+                    keep_for_capture(p)
                 pmask |= 1 << i
                 op.ptr[i] = p.data_ptr()
                 if p.dim() == 3 and p.shape[0] > 1:
@@ -359,6 +379,8 @@ class JonesOp:
             else:
                 op.sval[i] = float(p)
         for i, t in enumerate(self.ptrs):
+            if self.kind == _lib.OP_CMUL and t.dim() == 3 and 1 < t.shape[0] < batch:
+                raise ValueError(f"masks for {t.shape[0]} entries, a batch of {batch} fields")
             op.ptr[i] = 0 if t is None else t.data_ptr()
             if t is not None and t.dim() == 3 and t.shape[0] > 1:
                 pbstride = ny * nx
@@ -370,13 +392,14 @@ class JonesOp:
         op.pbstride = pbstride
 
 
-def fill_prog(prog: _lib.XlProg, ops, ny, nx) -> None:
+def fill_prog(prog: _lib.XlProg, ops, ny, nx, batch=1) -> None:
+    """``batch``: the fields of the launch; planes for fewer of them are refused."""
     ops = list(ops or ())
     if len(ops) > _lib.XL_MAX_OPS:
         raise ValueError(f"at most {_lib.XL_MAX_OPS} fused operations per pass")
     prog.nops = len(ops)
     for i, o in enumerate(ops):
-        o.fill(prog.ops[i], ny, nx)
+        o.fill(prog.ops[i], ny, nx, batch)
 
 
 def op_phase(phase):
@@ -453,7 +476,7 @@ def mask_planes(op, lead, ny, nx) -> torch.Tensor:
     B = int(np.prod(lead)) if len(lead) else 1
     out = torch.empty(tuple(lead) + (ny, nx), dtype=torch.complex64, device=device())
     prog = _lib.XlProg()
-    fill_prog(prog, [op], ny, nx)
+    fill_prog(prog, [op], ny, nx, B)
     _lib.check(lib().xl_mask_planes(stream_handle(), B, ny, nx, out.data_ptr(), ny * nx, ctypes.byref(prog)),
                "xl_mask_planes")
     return out
@@ -505,7 +528,7 @@ def apply_ops(comps, ops, ny, nx):
     comps, B, ibs = batch_planes(comps, ny, nx)
     outs = [torch.empty(tuple(lead) + (ny, nx), dtype=torch.complex64, device=comps[0].device) for _ in comps]
     prog = _lib.XlProg()
-    fill_prog(prog, ops, ny, nx)
+    fill_prog(prog, ops, ny, nx, B)
     inp = (ctypes.c_void_p * 3)(*[c.data_ptr() for c in comps] + [0] * (3 - len(comps)))
     out = (ctypes.c_void_p * 3)(*[o.data_ptr() for o in outs] + [0] * (3 - len(outs)))
     _lib.check(L.xl_apply_ops(stream_handle(), B, len(comps), ny, nx, inp, ibs, out, ny * nx,
@@ -532,28 +555,36 @@ def ops_backward(base, gout, ops, ny, nx, want_input=True):
            for i in range(C)]
     pgrad = (ctypes.c_void_p * (_lib.XL_MAX_OPS * 4))()
     grads = {}
-    scalars = []
+    scalars, shared = [], []
     for k, o in enumerate(ops):
         for q, p in enumerate(o.params):
             if isinstance(p, torch.Tensor):
                 if not p.requires_grad:
                     continue
+                nb = o.plane_batch()
                 if JonesOp.is_scalar_tensor(p):
-                    t = torch.empty(JonesOp.plane_shape(p, ny, nx), dtype=torch.float32, device=dev)
+                    shape = JonesOp.plane_shape(p, ny, nx)
                     scalars.append((k, q, p.shape))
                 else:
-                    t = torch.empty(p.shape, dtype=torch.float32, device=dev)
+                    shape = p.shape
+                if nb > 1 and math.prod(shape) == ny * nx:   # a plane shared by the batch beside planes per entry
+                    shared.append((k, q, shape))
+                    shape = (nb, ny, nx)
+                # planes past the batch get no gradient
+                t = (torch.zeros if nb > B else torch.empty)(shape, dtype=torch.float32, device=dev)
             else:
                 continue
             grads[(k, q)] = t
             pgrad[k * 4 + q] = t.data_ptr()
     prog = _lib.XlProg()
-    fill_prog(prog, ops, ny, nx)
+    fill_prog(prog, ops, ny, nx, B)
     inp = (ctypes.c_void_p * 3)(*[(b.data_ptr() if b is not None else 0) for b in base] + [0] * (3 - len(base)))
     go = (ctypes.c_void_p * 3)(*[(g.data_ptr() if g is not None else 0) for g in gout] + [0] * (3 - C))
     gi = (ctypes.c_void_p * 3)(*[(g.data_ptr() if g is not None else 0) for g in gin] + [0] * (3 - C))
     _lib.check(L.xl_ops_backward(stream_handle(), B, C, ny, nx, inp, ibs, go, ny * nx, gi, ny * nx,
                                  ctypes.byref(prog), pgrad), "xl_ops_backward")
+    for k, q, shape in shared:
+        grads[(k, q)] = grads[(k, q)][:B].sum(dim=0).reshape(shape)
     for k, q, shape in scalars:
         grads[(k, q)] = grads[(k, q)].sum(dim=(-2, -1)).reshape(shape)
     return gin, grads
@@ -765,8 +796,8 @@ class RsCall:
         a.spectrum_index = _ptr(spec_index)
         a.spectra = _ptr(spec_ptrs)
         a.work = work.data_ptr()
-        fill_prog(a.pre, pre, ny, nx)
-        fill_prog(a.post, post, ny, nx)
+        fill_prog(a.pre, pre, ny, nx, B)
+        fill_prog(a.post, post, ny, nx, B)
         a.adjoint = 1 if adjoint else 0
         self.args = a
         self.outs = outs
@@ -1124,7 +1155,7 @@ class CztCall:
             fin, fout = TRANSFER_PLANES.pair(x, y, xout, yout, zz, wavelength)
             if fin is not None:
                 a.f_in, a.f_out = fin.data_ptr(), fout.data_ptr()
-        fill_prog(a.pre, pre, ny, nx)
+        fill_prog(a.pre, pre, ny, nx, B)
         self.args = a
         self.outs = outs
         self._keep = (comps, work, prex, gx, postx, prey, gy, posty, gx_, gy_, gxo, gyo, list(pre or ()), zb, cteb,
