@@ -137,7 +137,7 @@ class _Fused(torch.autograd.Function):
         base = ctx.saved_tensors
         ref = next((g for g in gouts if g is not None), None)
         gouts = [g if g is not None else torch.zeros_like(ref) for g in gouts]
-        gouts = [g.to(torch.complex64).contiguous() for g in gouts]
+        gouts = [g.to(torch.complex64).resolve_conj().contiguous() for g in gouts]
         want_z = _z_tensor(plan) is not None and ctx.needs_input_grad[-1]
         gez = None
         if want_z and plan.vector:
@@ -185,7 +185,7 @@ class _Ops(torch.autograd.Function):
     def backward(ctx, *gouts):
         base = ctx.saved_tensors
         ref = next((g for g in gouts if g is not None), None)
-        gouts = [(g if g is not None else torch.zeros_like(ref)).to(torch.complex64).contiguous() for g in gouts]
+        gouts = [(g if g is not None else torch.zeros_like(ref)).to(torch.complex64).resolve_conj().contiguous() for g in gouts]
         want = any(t.requires_grad for t in base)
         gin, pgrads = engine.ops_backward(list(base), gouts, ctx.ops, ctx.ny, ctx.nx, want_input=want)
         trainable = _trainable(ctx.ops)

@@ -66,7 +66,10 @@ def _is_broadcast_batch(t: torch.Tensor) -> bool:
 def as_field(a, dev=None) -> torch.Tensor:
     """complex64 on the CUDA device, contiguous; a batch that is one plane
     broadcast along the batch (an ``expand``-ed view) stays a view, since
-    every launch takes it without copying (batch stride 0)."""
+    every launch takes it without copying (batch stride 0).  A lazily conjugated
+    tensor is conjugated in memory, which is what the kernels read."""
+    if isinstance(a, torch.Tensor):
+        a = a.resolve_conj()
     if isinstance(a, torch.Tensor) and a.is_cuda and a.dtype == torch.complex64 and dev is None:
         return a if (a.is_contiguous() or _is_broadcast_batch(a)) else a.contiguous()
     dev = dev or device()
@@ -86,7 +89,7 @@ def batch_planes(comps, ny, nx):
     A batch of fields that is one plane broadcast along the batch (an
     ``expand``-ed view, stride 0) is passed without copying, with batch stride 0.
     """
-    comps = [c if isinstance(c, torch.Tensor) else as_field(c) for c in comps]
+    comps = [c.resolve_conj() if isinstance(c, torch.Tensor) else as_field(c) for c in comps]
     lead = comps[0].shape[:-2]
     B = int(np.prod(lead)) if len(lead) else 1
     if B > 1 and all(c.dim() == 3 and c.stride(0) == 0 and c.dtype == torch.complex64 and c.is_cuda and
@@ -1437,7 +1440,7 @@ def _bs_args(a, b, m, ny, nx, kind=0):
             m = m[0]
         if m.dim() == 3 and m.shape[0] != B:
             raise ValueError(f"{m.shape[0]} splitter matrices for a batch of {B}")
-        m = m.to(torch.complex64).contiguous()
+        m = m.to(torch.complex64).resolve_conj().contiguous()
         args.m = m.data_ptr()
         args.m_bstride = 4 if m.dim() == 3 else 0
     else:
@@ -1505,7 +1508,7 @@ def _loss_planes(t: torch.Tensor):
     """(contiguous planes, count, plane stride, complex?) of a (..., ny, nx)
     complex64 field or float32 intensity."""
     cplx = t.is_complex()
-    t = (t.to(torch.complex64) if cplx else t.to(torch.float32)).contiguous()
+    t = (t.to(torch.complex64).resolve_conj() if cplx else t.to(torch.float32)).contiguous()
     ny, nx = t.shape[-2:]
     return t, t.numel() // (ny * nx), ny * nx, cplx
 
