@@ -68,7 +68,7 @@ def as_field(a, dev=None) -> torch.Tensor:
     broadcast along the batch (an ``expand``-ed view) stays a view, since
     every launch takes it without copying (batch stride 0).  A lazily conjugated
     tensor is conjugated in memory, which is what the kernels read."""
-    if isinstance(a, torch.Tensor):
+    if isinstance(a, torch.Tensor) and a.is_conj():
         a = a.resolve_conj()
     if isinstance(a, torch.Tensor) and a.is_cuda and a.dtype == torch.complex64 and dev is None:
         return a if (a.is_contiguous() or _is_broadcast_batch(a)) else a.contiguous()
@@ -89,15 +89,16 @@ def batch_planes(comps, ny, nx):
     A batch of fields that is one plane broadcast along the batch (an
     ``expand``-ed view, stride 0) is passed without copying, with batch stride 0.
     """
-    comps = [c.resolve_conj() if isinstance(c, torch.Tensor) else as_field(c) for c in comps]
+    comps = [c if isinstance(c, torch.Tensor) else as_field(c) for c in comps]
     lead = comps[0].shape[:-2]
     B = int(np.prod(lead)) if len(lead) else 1
     if B > 1 and all(c.dim() == 3 and c.stride(0) == 0 and c.dtype == torch.complex64 and c.is_cuda and
                      c[0].is_contiguous() for c in comps):
-        return [c[0] for c in comps], B, 0
+        return [c[0].resolve_conj() for c in comps], B, 0
     planes = [as_field(c).contiguous() for c in comps]
-    if any(p.numel() < B * ny * nx for p in planes):
-        raise ValueError(f"components of shapes {[tuple(p.shape) for p in planes]} in a batch of {B} fields")
+    for p in planes[1:]:
+        if p.numel() < B * ny * nx:
+            raise ValueError(f"components of shapes {[tuple(c.shape) for c in planes]} in a batch of {B} fields")
     return planes, B, ny * nx
 
 
@@ -188,8 +189,8 @@ def is_plain_cuda(t) -> bool:
     miss the kernel that fills it)."""
     if torch.compiler.is_compiling():
         return False
-    return (type(t) in (torch.Tensor, torch.nn.Parameter) and not torch.jit.is_tracing() and
-            not torch._C._len_torch_dispatch_stack() and t.is_cuda and
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and
+            torch._C._get_tracing_state() is None and not torch._C._len_torch_dispatch_stack() and
             t.device.index == torch.cuda.current_device() and not t.is_neg() and
             not torch._C._functorch.is_functorch_wrapped_tensor(t))
 
@@ -319,7 +320,7 @@ def quality_factor(x, y, wavelength, z):
 class JonesOp:
     """One per-pixel operation of a fused program (see XL_OP_* in xlgb.h)."""
 
-    __slots__ = ("kind", "params", "ptrs", "sval", "dval", "keep", "planes", "copies")
+    __slots__ = ("kind", "params", "ptrs", "sval", "dval", "keep", "planes", "copies", "nb")
 
     def __init__(self, kind, params=(), ptrs=(), sval=(), dval=(), keep=()):
         self.kind = kind
@@ -330,6 +331,7 @@ class JonesOp:
         self.keep = list(keep)
         self.planes = {}             # slot -> plane a one-element tensor parameter was expanded to
         self.copies = {}             # slot -> the last launch's copies of a plane shared by the batch
+        self.nb = 0                  # plane_batch's result, once asked for
 
     @staticmethod
     def is_scalar_tensor(p) -> bool:
@@ -347,17 +349,22 @@ class JonesOp:
         """Planes per parameter: the batch of those that have one for every entry,
         1 if all are shared by it.  An op has one stride for all of them, so a
         shared plane beside them is copied for every entry."""
-        sizes = {p.numel() if p.dim() < 2 else p.shape[0] for p in self.params
-                 if isinstance(p, torch.Tensor) and (p.dim() == 3 or p.dim() < 2)} - {1}
-        if len(sizes) > 1:
-            raise ValueError(f"mask parameters of one device have batches of {sorted(sizes)} planes")
-        return sizes.pop() if sizes else 1
+        if not self.nb:
+            nb = 1
+            for p in self.params:
+                if isinstance(p, torch.Tensor) and p.dim() != 2 and p.dim() < 4:
+                    n = p.shape[0] if p.dim() == 3 else p.numel()
+                    if n not in (1, nb) and nb > 1:
+                        raise ValueError(f"mask parameters of one device have batches of {nb} and {n} planes")
+                    nb = max(nb, n)
+            self.nb = nb
+        return self.nb
 
     def fill(self, op: _lib.XlOp, ny: int, nx: int, batch: int = 1) -> None:
         op.kind = self.kind
         pmask = 0
         pbstride = 0
-        nb = self.plane_batch()
+        nb = self.nb or self.plane_batch()
         if 1 < nb < batch:
             raise ValueError(f"mask parameters for {nb} entries, a batch of {batch} fields")
         for i, p in enumerate(self.params):
